@@ -270,7 +270,7 @@ void upload_scene(nr_scene* s) {
     }
 
     // The same nodes with every child box widened by delta for the one-FMA
-    // box test without margin (traversal mode 2). For a ray origin o with
+    // box test without margin (fast_box). For a ray origin o with
     // |o_i| <= Bo and box bounds b with |b_i| <= A, the test's quotient
     // fma(b, 1/d, -o/d) and the reference's RN(RN(b - o) / d) each lie within
     // 2^-23 (|b| + |o|) / |d| of (b - o) / d, so widening by more than
@@ -286,11 +286,13 @@ void upload_scene(nr_scene* s) {
             E = std::max(E, 0.5f * (B.nodes[0].hi[k] - B.nodes[0].lo[k]));
         }
     const float delta = 4e-6f * (A + E) + 1e-30f;
-    std::vector<nr::GpuNode> gf(gn);
-    for (auto& g : gf) {
-        g.a = make_float4(g.a.x - delta, g.a.y + delta, g.a.z - delta, g.a.w + delta);
-        g.b = make_float4(g.b.x - delta, g.b.y + delta, g.b.z - delta, g.b.w + delta);
-        g.c = make_float4(g.c.x - delta, g.c.y + delta, g.c.z - delta, g.c.w + delta);
+    std::vector<nr::FastNode> gf(ng);
+    for (int i = 0; i < ng; ++i) {
+        const nr::GpuNode& g = gn[i];
+        gf[i] = nr::FastNode{{g.a.x - delta, g.a.z - delta, g.a.y + delta, g.a.w + delta, g.c.x - delta, g.c.y + delta},
+                             {g.d.x, g.d.y},
+                             {g.b.x - delta, g.b.z - delta, g.b.y + delta, g.b.w + delta, g.c.z - delta, g.c.w + delta},
+                             {0, 0}};
     }
 
     // emitters in loader order, weight = Triangle::area (twice the area)
@@ -367,7 +369,7 @@ void upload_scene(nr_scene* s) {
 
     nr::DeviceScene& D = s->dev;
     D.nodes = s->nodes.as<nr::GpuNode>();
-    D.nodes_fast = s->nodes_fast.as<nr::GpuNode>();
+    D.nodes_fast = s->nodes_fast.as<nr::FastNode>();
     D.fast_origin_bound = 2.0f * A + 4.0f * E;
     D.tri_geo = s->tri_geo.as<float4>();
     D.tri_shade = s->tri_shade.as<float4>();

@@ -84,74 +84,39 @@ __device__ __forceinline__ void warp_count(uint32_t v, uint32_t* lohi) {
 }
 
 // Closest hit, persistent: warps take 32 queue entries at a time from a
-// shared cursor, one ray per lane to completion (closest_hit), then the slot
-// is bucketed by shading category (material type of the hit, or CAT_MISS).
-// FAST (trav=1) walks the widened boxes with the one-FMA test alone and
-// tests triangles with the fast test and its exact fallback; !FAST (trav=0)
-// walks the reference's boxes with its exact arithmetic. The widened boxes
-// accept every box the exact test accepts, so trav=1 reaches every triangle
-// trav=0 reaches (the same hits but where a ray passes within about 1e-6 of
-// a box face and hits a triangle there that the exact test's rounding
-// excludes). Measured on the 1M-triangle frame: 757.5 Mpaths/s with the
-// margin-and-fallback box test on the reference's boxes, 866.4 with the
-// one-FMA test alone (not conservative), 831.3 with that test widened by its
-// error bound at run time. (Measured and dropped: a variant that
-// refilled idle lanes from the queue with separate node and leaf phases,
-// 28 % slower; a four-wide tree collapsed from this one, no faster.)
+// shared cursor, one ray per lane to completion, then the slot is bucketed by
+// shading category (material type of the hit, or CAT_MISS).
+// FAST (trav=1) walks the widened boxes (closest_hit_fast); !FAST (trav=0)
+// the reference's boxes with its exact arithmetic (closest_hit_ww). The
+// widened boxes accept every box the exact test accepts, so trav=1 reaches
+// every triangle trav=0 reaches (the same hits but where a ray passes within
+// about 1e-6 of a box face and hits a triangle there that the exact test's
+// rounding excludes). Measured and dropped: refilling idle lanes from the
+// queue with separate node and leaf phases, 28 % slower; a four-wide tree of
+// these boxes (128-byte nodes, sorted children): half the visits but as many
+// L1 wavefronts and more issue slots a visit, 147 against 136 ms a frame; a
+// warp walking one shared stack for its 32 shadow rays, 61 against 30 ms even
+// on rays sorted by origin and direction.
 // Minimum resident 128-thread blocks per SM requested from the register
-// allocator for the two traversal kernels (NR_TRACE_MINB, NR_SHADOW_MINB
-// below). Traversal is bound by dependent L2 latency, so extra warps pay:
-// measured on GB300 for the 1M-triangle frame with the if-if loops, 566
-// Mpaths/s at 10 blocks (48 registers, 40 warps) against 530 with no cap
-// (53 registers, 36 warps) and 541 at 12 (40 registers, with spills); the
-// current loops and caps below.
-// Loop shape (NR_WW bits): 1 closest hit while-while with postponed leaves
-// (closest_hit_ww), 8 the same without postponing; 2 / 4 any hit likewise;
-// 0 the if-if loops (closest_hit, any_hit). Measured for the 1M-triangle
-// frame: if-if 585.5 Mpaths/s; postponed leaves in both 591.9 (k_trace
-// -14 %, k_shadow slower: its first leaf often holds the occluder); in
-// closest hit only 636.6; with any hit while-while without postponing 645.4;
-// closest hit without postponing too 606.6. With this shape the caps were
-// best at 10 / 10 (trace 8: 621.8, 12: 629.6; shadow 8: 639.9, 12: 603.1).
-// Once the closest-hit walk lost its step budget (one register less) and
-// took the folded box test, 12 blocks (40 registers, 28 bytes of spills)
-// overtook 10 for it: 912.2 against 901.4 Mpaths/s, 9 blocks 879.9; the
-// shadow kernel stays at 10 (8: 906.8, 12: 909.7, 10: 912.1).
-// Also measured and dropped for the shadow rays: dynamic fetch of new rays
-// into idle lanes (Aila and Laine 2009) at 4, 8 or 16 idle lanes, 571;
-// the shadow queue sorted by light (counting sort, 257 buckets) before the
-// shadow kernel, 541: rays from neighbouring pixels to different lights
-// share more of their walk than rays to one light from across the frame.
-// Likewise within a warp's window of 128 or 256 queued rays, grouped by the
-// cell of a 4x4x4 grid holding the ray's end point (counting sort in shared
-// memory): 756.1 and 743.3 against 772.1.
+// allocator for the two traversal kernels. 1M-triangle frame of 1080p x 64
+// spp, ms: closest hit at 8 / 10 / 12 blocks 79.2 / 76.6 / 73.2 (40 registers,
+// 84 bytes of spills at 12); shadow rays at 8 / 10 / 12 42.7 / 42.9 / 42.5.
+// Loop shape: closest hit while-while with postponed leaves, any hit without
+// (its first leaf often holds the occluder): 645.4 Mpaths/s against 591.9
+// with postponed leaves in both and 606.6 without in either. Also measured
+// and dropped for the shadow rays: dynamic fetch of new rays into idle lanes
+// (Aila and Laine 2009) at 4, 8 or 16 idle lanes, 571.
 #ifndef NR_TRACE_MINB
 #define NR_TRACE_MINB 12
 #endif
 #ifndef NR_SHADOW_MINB
 #define NR_SHADOW_MINB 10
 #endif
-#ifndef NR_WW
-#define NR_WW 5
-#endif
-// Entries of each traversal stack kept in shared memory (a power of two; 0:
-// all in local memory). Measured on the 1M-triangle frame: K = 4 704.2 and
-// K = 8 706.1 against 757.5 Mpaths/s with the whole stack in local memory
-// (L1-resident already; the ring's index arithmetic costs issue slots).
-#ifndef NR_SMEM_STACK
-#define NR_SMEM_STACK 0
-#endif
-
 template <bool COUNT, bool FAST>
 __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, DeviceScene S, int capacity) {
     const uint32_t n = P.counters[CNT_IN];
     const int lane = threadIdx.x & 31;
     uint32_t nv = 0, nt = 0;
-#if NR_SMEM_STACK
-    __shared__ int2 ring[NR_SMEM_STACK * 128];
-#else
-    int2* ring = nullptr;
-#endif
     while (true) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&P.counters[CNT_WORK], 32u);
@@ -162,11 +127,8 @@ __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, Devic
             int slot = P.queue_in[idx];
             f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
             float t, b1, b2;
-            int tri = (NR_WW & 9) ? closest_hit_ww<FAST ? 2 : 0, (NR_WW & 1) != 0, NR_SMEM_STACK>(
-                                        S, o, d, t, b1, b2, &P.counters[CNT_ERR], COUNT ? &nv : nullptr,
-                                        COUNT ? &nt : nullptr, ring)
-                            : closest_hit<FAST>(S, o, d, t, b1, b2, &P.counters[CNT_ERR], COUNT ? &nv : nullptr,
-                                                COUNT ? &nt : nullptr);
+            const int tri = FAST ? closest_hit_fast(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr)
+                                 : closest_hit_ww(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
             int cat = CAT_MISS;
             if (tri >= 0) cat = S.mats[__float_as_int(__ldg(&S.tri_geo[3 * tri + 1]).w)].type;
@@ -202,11 +164,6 @@ __global__ void __launch_bounds__(128, NR_SHADOW_MINB) k_shadow(PathState P, Dev
     const uint32_t n = min(P.counters[CNT_SHADOW], (uint32_t)P.sh_cap);
     const int lane = threadIdx.x & 31;
     uint32_t nv = 0, nt = 0;
-#if NR_SMEM_STACK
-    __shared__ int ring[NR_SMEM_STACK * 128];
-#else
-    int* ring = nullptr;
-#endif
     while (true) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&P.counters[CNT_WORK_SH], 32u);
@@ -218,11 +175,9 @@ __global__ void __launch_bounds__(128, NR_SHADOW_MINB) k_shadow(PathState P, Dev
             const bool env = o.w < 0.f;  // an environment sample: k_env_fold adds it
             const float tmax = env ? -o.w : o.w;
             const bool occluded =
-                (NR_WW & 6) ? any_hit_ww<FAST ? 2 : 0, (NR_WW & 2) != 0, NR_SMEM_STACK>(
-                                  S, xyz(o), xyz(d), tmax, &P.counters[CNT_ERR], COUNT ? &nv : nullptr,
-                                  COUNT ? &nt : nullptr, ring)
-                      : any_hit<FAST>(S, xyz(o), xyz(d), tmax, &P.counters[CNT_ERR], COUNT ? &nv : nullptr,
-                                      COUNT ? &nt : nullptr);
+                FAST ? any_hit_fast(S, xyz(o), xyz(d), tmax, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr)
+                     : any_hit_ww<false>(S, xyz(o), xyz(d), tmax, &P.counters[CNT_ERR], COUNT ? &nv : nullptr,
+                                         COUNT ? &nt : nullptr);
             if (P.vis) P.vis[__float_as_int(d.w)] = occluded ? 0 : 1;
             if (env) {
                 if (occluded) P.sh_c[idx].x = P.sh_c[idx].y = P.sh_c[idx].z = 0.f;
@@ -277,18 +232,18 @@ __device__ __forceinline__ bool nrc_is_training(uint32_t pixel, uint32_t sample,
 // Queues a shadow ray (or, when no hit can come before the limit, adds its
 // contribution at once). rec: the training record whose target leaves this
 // light sample out, or -1.
-// TAIL: trace the shadow ray here (the any-hit walk of k_shadow) instead of
+// TAIL: trace the shadow ray here (1: exact walk, 2: fast) instead of
 // queueing it. env: the vertex's environment sample, queued with its limit
 // negated: k_shadow leaves its contribution in the queue entry (zero when
 // occluded) and k_env_fold adds it after the area-light samples, so each
 // path's radiance has one writer at a time and the restatement's order.
-template <bool NRC, bool TAIL = false>
+template <bool NRC, int TAIL = 0>
 __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScene& S, const Policy& pol,
                                             const NrcCtx& C, int slot, int rec, f3 so, f3 d, float tmax, f3 c,
                                             bool env = false) {
     if (TAIL && tmax > 0.f) {
-        const bool occluded = pol.trav ? any_hit_ww<2, (NR_WW & 2) != 0>(S, so, d, tmax, &P.counters[CNT_ERR])
-                                       : any_hit_ww<0, (NR_WW & 2) != 0>(S, so, d, tmax, &P.counters[CNT_ERR]);
+        const bool occluded = TAIL == 2 ? any_hit_fast(S, so, d, tmax)
+                                        : any_hit_ww<false>(S, so, d, tmax, &P.counters[CNT_ERR]);
         if (occluded) return;
         tmax = 0.f;  // unoccluded: added below
     }
@@ -309,9 +264,10 @@ __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScen
 }
 
 // MT: the shading category when it is known at compile time (a material
-// type, or CAT_MISS), -1 for any. TAIL: light samples traced here and the
-// continuing path not queued. Returns whether the path goes on.
-template <bool NRC, int MT = -1, bool TAIL = false>
+// type, or CAT_MISS), -1 for any. TAIL: light samples traced here (1 by the
+// exact walk, 2 by the fast one) and the continuing path not queued. Returns
+// whether the path goes on.
+template <bool NRC, int MT = -1, int TAIL = 0>
 __device__ __forceinline__ bool shade_one(const PathState& P, const DeviceScene& S, const Policy& pol, int slot,
                                           const NrcCtx& C) {
     float4 h = P.hit[slot];
@@ -568,9 +524,9 @@ __global__ void __launch_bounds__(128, NR_TAIL_MINB) k_tail(PathState P, DeviceS
     for (int b = 0; b < NR_TAIL_MAX_BOUNCES; ++b) {
         const f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
         float t, b1, b2;
-        const int tri = closest_hit_ww<FAST ? 2 : 0>(S, o, d, t, b1, b2, &P.counters[CNT_ERR]);
+        const int tri = FAST ? closest_hit_fast(S, o, d, t, b1, b2) : closest_hit_ww(S, o, d, t, b1, b2);
         P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
-        if (!shade_one<NRC, -1, true>(P, S, pol, slot, C)) return;
+        if (!shade_one<NRC, -1, FAST ? 2 : 1>(P, S, pol, slot, C)) return;
     }
     atomicOr(&P.counters[CNT_ERR], 16u);  // bounce cap: the path did not end
 }

@@ -34,6 +34,16 @@ struct alignas(16) GpuNode {
     int4 d;
 };
 
+// The same node as the fast walk (trav=1) reads it, 64 bytes, with the boxes
+// widened (upload_scene): one 32-byte load per child, bounds in the pairs that
+// the two-wide FMA takes. c = (lo.x, lo.y, hi.x, hi.y, lo.z, hi.z).
+struct alignas(64) FastNode {
+    float c0[6];
+    int32_t ref[2];
+    float c1[6];
+    int32_t pad[2];
+};
+
 // Per flattened triangle, traversal data, 48 bytes:
 //   g0 = (p0.xyz, loader index bits), g1 = (e1.xyz, material bits), g2 = (e2.xyz, 0)
 // with e1 = p1 - p0 and e2 = p2 - p0 rounded exactly as the reference does.
@@ -67,8 +77,8 @@ struct DeviceScene {
     int32_t max_depth;        // deepest leaf (root = 0)
     int32_t num_nodes;        // internal nodes
     float prune_k;            // subtrees entered beyond prune_k x the best hit are skipped (infinity: none)
-    const GpuNode* nodes_fast;  // the same nodes with every box widened for box_test_plain (traversal mode 2)
-    float fast_origin_bound;    // mode 2 is conservative for ray origins with every |coordinate| <= this
+    const FastNode* nodes_fast;  // the same nodes with every box widened, for the fast walk (trav=1)
+    float fast_origin_bound;     // the fast walk is conservative for ray origins with every |coordinate| <= this
 };
 
 // Render policy decoded from the parameter string.
