@@ -293,9 +293,11 @@ int nr_intersect_noalloc(nr_scene* scene, int32_t n, const float* o, const float
  * 0 and imgh % 4 == 0; else or with 0: scanline order), live_sync (with
  * maxdepth: the bounce after which the live path count is read back each
  * bounce; -1, the default, 5 for waves of more than 2^22 paths and never
- * for smaller ones), tail (waves of at most 2^22 paths: after this many
- * wavefront bounces one launch takes every live path to its end, tracing
- * its light samples inline; default 2, 0 never; the image is the same),
+ * for smaller ones), tail (when
+ * one launch takes every live path to its end, tracing its light samples
+ * inline: -1, the default, once a bounce starts with few paths; N > 0, in
+ * waves of at most 2^22 paths after N wavefront bounces; 0 never; the image
+ * is the same),
  * prune (1, the default: a traversal skips subtrees entered beyond 1.001 x
  * its best hit so far or its shadow ray's length; 0: every node whose box a
  * ray enters is visited, as the reference's exhaustive BVH::_traversal, for

@@ -157,7 +157,8 @@ struct nr_scene {
     nr::PathState ps{};
     int capacity = 0;
     int sh_mult = 1;  // shadow-ray queue entries per path slot
-    uint32_t* counters_host = nullptr;  // pinned
+    uint32_t* counters_host = nullptr;  // pinned: the counters, then two live counts in flight
+    cudaEvent_t live_ev[2] = {nullptr, nullptr};  // their arrival
     nr_stats stats{};
     std::vector<cudaEvent_t> ev_pool;  // profile=1: events around every kernel group
     nr_nrc* nrc = nullptr;             // attached cache (not owned)
@@ -186,6 +187,8 @@ struct nr_scene {
         for (auto* b : all_bufs()) b->release();
         if (counters_host) cudaFreeHost(counters_host);
         for (auto& e : ev_pool) cudaEventDestroy(e);
+        for (auto& e : live_ev)
+            if (e) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -421,7 +424,8 @@ void finish_scene(nr_scene* s, const char* options, nr::Bvh* prebuilt = nullptr)
     NR_CUDA(cudaGetDevice(&s->device));
     NR_CUDA(cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, s->device));
     NR_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    NR_CUDA(cudaMallocHost(&s->counters_host, nr::NUM_COUNTERS * sizeof(uint32_t)));
+    NR_CUDA(cudaMallocHost(&s->counters_host, (nr::NUM_COUNTERS + 2) * sizeof(uint32_t)));
+    for (auto& e : s->live_ev) NR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     auto t0 = std::chrono::steady_clock::now();
     s->bvh_device_ms = 0.0;
     // the deepest tree the traversal stacks hold; the builders stop past it
@@ -594,10 +598,9 @@ struct RenderArgs {
     // against 699.0 without; 960x540 frames of 1 spp 2.789 ms with it,
     // 2.735 without (the wait costs more than the grid saves).
     int live_sync;
-    // Small waves (at most 2^22 paths): the wavefront bounces after which
-    // k_tail takes every live path to its end in one launch (0: never).
-    // 960x540 frames of 1 spp on the 1M-triangle scene: 2.557 ms without,
-    // 2.305 / 1.805 / 1.821 / 2.046 ms after 1 / 2 / 3 / 4 bounces.
+    // When k_tail takes every live path to its end in one launch: -1, the
+    // default, by the live count (tail_limit); N > 0: in waves of at most 2^22
+    // paths after N wavefront bounces; 0: never.
     int tail;
     bool nrc;
     int nrc_train;    // training paths per wavefront batch
@@ -682,7 +685,7 @@ RenderArgs parse_args(const nr_camera* cam, const char* params) {
     a.tile = c.get_int("tile", 2);
     if (a.tile < 0 || a.tile > 2) throw NrError(NR_ERR_INVALID, "tile must be 0, 1 or 2");
     a.live_sync = c.get_int("live_sync", -1);
-    a.tail = c.get_int("tail", 2);
+    a.tail = c.get_int("tail", -1);
     // 0: the largest power of two up to 32 that divides spp
     a.tile_samples = c.get_int("tile_samples", 0);
     if (a.tile_samples < 0 || a.tile_samples > 32 || (a.tile_samples & (a.tile_samples - 1)))
@@ -767,6 +770,18 @@ void wave_layout(const RenderArgs& A, bool has_pix_list, nr::WaveDesc& W) {
 // NR_TAIL_MAX_BOUNCES too): paths end by Russian roulette, misses and
 // emitters, but prr = 1 in a closed scene would never end.
 constexpr int kMaxBounces = 4096;
+// Paths entering a bounce at or below which the tail kernel takes them all to
+// their end. Its warps shade whatever material each lane met, so the line
+// lies lower where several surface types occur, and lower still for a whole
+// wave, whose bounces mostly lie ahead. ms with the line below / above the
+// count, 1M triangles of one type: 230k paths 1.12 / 0.77, 518k 1.55 / 1.35,
+// 1.04M 2.12 / 2.35; every type, unbounded paths: 246k 0.64 / 0.60, 522k 0.76 /
+// 0.97; a room of four types: 246k 0.94 / 1.26, 1.04M with 1.75 from 150k on,
+// 2.52 from 600k on; sky and dielectrics, 518k 1.70 / 2.02.
+int64_t tail_limit(uint32_t cat_mask, int bounce) {
+    const int surfaces = __builtin_popcount(cat_mask & ((1u << NR_MAT_LIGHT) - 1u));
+    return surfaces <= 1 ? 600000 : (bounce == 0 ? 200000 : 300000);
+}
 
 void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pix, int sample0, float4* film,
                float* dev_out, volatile int32_t* cancel, void (*progress)(float, void*), void* user) {
@@ -863,13 +878,23 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
         nr::launch_raygen(P, W, A.cam, film_h, A.pol, st);
         S.kernel_launches += 2;
         mark(3);
-        int live = W.count;
-        const bool tail = A.tail > 0 && cap <= nr::SHADE_SPLIT_MIN && !A.profile && !A.count;
+        // The tail kernel from the first bounce known to start with few paths:
+        // by the wave's size, later by the live counts, which the host reads one
+        // bounce behind so that the device always has a bounce queued. An
+        // explicit tail=N stands for waves of at most 2^22 paths.
+        const bool stepwise = A.profile || A.count;  // these time or count the wavefront's own kernels
+        // (Waves of more than 2^25 paths and bounded depth: their last bounces
+        // are under 1 % of them, 140.3 against 140.4 ms, and stay as they are.)
+        const int tail_at = A.tail > 0 ? (cap <= nr::SHADE_SPLIT_MIN ? A.tail : kMaxBounces)
+                            : (A.tail < 0 && (cap <= (1 << 25) || A.pol.maxdepth == 0) ? -1 : kMaxBounces);
+        int live = W.count;     // an upper bound of the paths entering the bounce
+        int reads = 0, taken = 0;  // live counts asked for and received
         for (int bounce = 0;; ++bounce) {
             if (A.pol.maxdepth > 0 && bounce >= A.pol.maxdepth) break;
             if (bounce >= kMaxBounces) throw NrError(NR_ERR_DEVICE, "paths still alive after 4096 bounces (prr = 1?)");
-            if (tail && bounce >= A.tail) {
-                nr::launch_tail(P, D, A.pol, cap, use_nrc ? &s->nrc_ctx : nullptr, st);
+            if (live == 0) break;
+            if (!stepwise && (tail_at >= 0 ? bounce >= tail_at : live <= tail_limit(s->dev.cat_mask, bounce))) {
+                nr::launch_tail(P, D, A.pol, live, use_nrc ? &s->nrc_ctx : nullptr, st);
                 S.kernel_launches += 1;
                 break;
             }
@@ -890,13 +915,19 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
             S.bounces++;
             S.trace_launches++;
             S.kernel_launches += nr::bounce_launches(cap, A.pol.envis != 0, s->dev.cat_mask);
-            // With a depth limit the loop runs exactly maxdepth bounces; without
-            // one the live count is read back to find the end of the wave.
-            if (A.pol.maxdepth == 0 || (live_sync > 0 && bounce + 1 >= live_sync)) {
-                NR_CUDA(cudaMemcpyAsync(s->counters_host, s->ps.counters, nr::NUM_COUNTERS * 4, cudaMemcpyDeviceToHost, st));
-                NR_CUDA(cudaStreamSynchronize(st));
-                live = (int)s->counters_host[nr::CNT_IN];
-                if (live == 0) break;
+            // The count entering the next bounce, read back; the one asked for
+            // a bounce earlier is taken now, while this bounce runs.
+            const bool last = A.pol.maxdepth > 0 && bounce + 1 >= A.pol.maxdepth;
+            if (!last && (A.pol.maxdepth == 0 || (tail_at < 0 && !stepwise) || (live_sync > 0 && bounce + 1 >= live_sync))) {
+                NR_CUDA(cudaMemcpyAsync(&s->counters_host[nr::NUM_COUNTERS + (reads & 1)], s->ps.counters + nr::CNT_IN, 4,
+                                        cudaMemcpyDeviceToHost, st));
+                NR_CUDA(cudaEventRecord(s->live_ev[reads & 1], st));
+                ++reads;
+                while (taken < reads - (A.pol.maxdepth == 0 && stepwise ? 0 : 1)) {
+                    NR_CUDA(cudaEventSynchronize(s->live_ev[taken & 1]));
+                    live = (int)s->counters_host[nr::NUM_COUNTERS + (taken & 1)];
+                    ++taken;
+                }
             }
         }
         if (use_nrc) {

@@ -8,6 +8,8 @@
 // (src/renderer/rendererptls.cpp:13-94) unrolled into an iteration:
 //   L += T * (NEE term);  T *= |wi.n| f / pdf / prr;  emitter hit: L += T * Ke * fac
 // which is the reference's recursion result = NEE + Li * |wi.n| f / pdf / prr.
+#include <algorithm>
+
 #include "nr_material.cuh"
 #include "integrator.h"
 
@@ -240,8 +242,9 @@ __device__ __forceinline__ bool nrc_is_training(uint32_t pixel, uint32_t sample,
 template <bool NRC, int TAIL = 0>
 __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScene& S, const Policy& pol,
                                             const NrcCtx& C, int slot, int rec, f3 so, f3 d, float tmax, f3 c,
-                                            bool env = false) {
+                                            uint32_t* shadows, bool env = false) {
     if (TAIL && tmax > 0.f) {
+        ++*shadows;
         const bool occluded = TAIL == 2 ? any_hit_fast(S, so, d, tmax)
                                         : any_hit_ww<false>(S, so, d, tmax, &P.counters[CNT_ERR]);
         if (occluded) return;
@@ -254,11 +257,13 @@ __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScen
         P.sh_d[q] = make_float4(d.x, d.y, d.z, __int_as_float(slot));
         P.sh_c[q] = make_float4(c.x, c.y, c.z, __int_as_float(rec));
     } else {
+        // c rounded before it is added, as k_shadow adds it from the queue: the
+        // same image whichever kernel takes a bounce
         float4 r = P.rad[slot];
-        P.rad[slot] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.f);
+        P.rad[slot] = make_float4(radd(r.x, c.x), radd(r.y, c.y), radd(r.z, c.z), 0.f);
         if (NRC && rec >= 0) {
             float4 b = C.t_before[rec];
-            C.t_before[rec] = make_float4(b.x + c.x, b.y + c.y, b.z + c.z, 0.f);
+            C.t_before[rec] = make_float4(radd(b.x, c.x), radd(b.y, c.y), radd(b.z, c.z), 0.f);
         }
     }
 }
@@ -269,7 +274,7 @@ __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScen
 // whether the path goes on.
 template <bool NRC, int MT = -1, int TAIL = 0>
 __device__ __forceinline__ bool shade_one(const PathState& P, const DeviceScene& S, const Policy& pol, int slot,
-                                          const NrcCtx& C) {
+                                          const NrcCtx& C, uint32_t* shadows = nullptr) {
     float4 h = P.hit[slot];
     float4 thr = P.thr[slot];
     uint4 meta = P.meta[slot];
@@ -388,7 +393,7 @@ __device__ __forceinline__ bool shade_one(const PathState& P, const DeviceScene&
             // double there), i.e. occluded iff some hit has t <= |lv| - 2e-3.
             double lim = (double)norm(light_vec) - 2e-3;
             float tmax = lim > 0.0 ? __double2float_rd(lim) : 0.0f;
-            emit_shadow<NRC, TAIL>(P, S, pol, C, slot, rec, hit_pos + wl * 1e-3f, wl, tmax, c);
+            emit_shadow<NRC, TAIL>(P, S, pol, C, slot, rec, hit_pos + wl * 1e-3f, wl, tmax, c, shadows);
         }
     }
     // envis: one environment light sample more (no counterpart in the
@@ -408,7 +413,7 @@ __device__ __forceinline__ bool shade_one(const PathState& P, const DeviceScene&
                 const float pb = last ? 0.f : mat_pdf(M, wo, normal, we);
                 const f3 c = T * mat_bxdf(M, wo, normal, we) * env_lookup(S, we) * (cosn / (pe + pb));
                 if (c.x != 0.f || c.y != 0.f || c.z != 0.f)
-                    emit_shadow<NRC, TAIL>(P, S, pol, C, slot, rec, hit_pos + we * 1e-3f, we, 3.0e38f, c, true);
+                    emit_shadow<NRC, TAIL>(P, S, pol, C, slot, rec, hit_pos + we * 1e-3f, we, 3.0e38f, c, shadows, true);
             }
         }
     }
@@ -500,9 +505,9 @@ static void launch_shade(const PathState& P, const DeviceScene& S, const Policy&
 
 // The rest of every live path in one launch, one thread per path: closest
 // hit, then shade_one in its TAIL form (light samples traced inline), until
-// the path ends. For small waves, whose last bounces hold few rays: the
-// bounce-by-bounce wavefront waits at each bounce for its slowest ray, this
-// kernel only for the slowest path. Same functions, same results.
+// the path ends. For bounces of few paths (run_waves decides): the wavefront
+// waits at each bounce for its slowest ray in each of its kernels, this kernel
+// only for the slowest path. Same functions, same results.
 #ifndef NR_TAIL_MAX_BOUNCES
 #define NR_TAIL_MAX_BOUNCES 4096
 #endif
@@ -515,20 +520,39 @@ static void launch_shade(const PathState& P, const DeviceScene& S, const Policy&
 #ifndef NR_TAIL_MINB
 #define NR_TAIL_MINB 8
 #endif
+// Paths of a warp: a warp walks for as long as its slowest ray in every
+// phase, so a few paths are spread over 16 warps per SM, and up to 8 warps
+// per SM before warps fill (the whole path in this kernel, 1M triangles, 3072
+// paths: 350 us with full warps, 263 / 238 / 227 / 214 over 4 / 8 / 16 / 32
+// warps per SM; 15,360 paths 354 / 314 / 289 / 315; the room of 36 triangles,
+// bound by issue slots at 61,440 paths: 510 / 509 / 570 / 633).
+#define NR_TAIL_WARPS 16
+__host__ __device__ inline uint32_t tail_paths_per_warp(uint32_t n, uint32_t sms) {
+    const uint32_t wide = sms * NR_TAIL_WARPS, warps = n <= 8u * wide ? wide : wide / 2u;
+    const uint32_t take = (n + warps - 1u) / warps;
+    return take < 1u ? 1u : (take > 32u ? 32u : take);
+}
 template <bool NRC, bool FAST>
-__global__ void __launch_bounds__(128, NR_TAIL_MINB) k_tail(PathState P, DeviceScene S, Policy pol, NrcCtx C) {
-    const uint32_t n = P.counters[CNT_IN];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int slot = P.queue_in[i];
-    for (int b = 0; b < NR_TAIL_MAX_BOUNCES; ++b) {
-        const f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
-        float t, b1, b2;
-        const int tri = FAST ? closest_hit_fast(S, o, d, t, b1, b2) : closest_hit_ww(S, o, d, t, b1, b2);
-        P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
-        if (!shade_one<NRC, -1, FAST ? 2 : 1>(P, S, pol, slot, C)) return;
+__global__ void __launch_bounds__(128, NR_TAIL_MINB) k_tail(PathState P, DeviceScene S, Policy pol, NrcCtx C,
+                                                              uint32_t sms) {
+    const uint32_t n = P.counters[CNT_IN], take = tail_paths_per_warp(n, sms);
+    const uint32_t lane = threadIdx.x & 31u, i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
+    uint32_t rays = 0, shadows = 0;
+    if (lane < take && i < n) {
+        const int slot = P.queue_in[i];
+        bool on = true;
+        for (int b = 0; on && b < NR_TAIL_MAX_BOUNCES; ++b) {
+            const f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
+            float t, b1, b2;
+            const int tri = FAST ? closest_hit_fast(S, o, d, t, b1, b2) : closest_hit_ww(S, o, d, t, b1, b2);
+            P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
+            ++rays;
+            on = shade_one<NRC, -1, FAST ? 2 : 1>(P, S, pol, slot, C, &shadows);
+        }
+        if (on) atomicOr(&P.counters[CNT_ERR], (uint32_t)NR_ERRBIT_BOUNCES);  // bounce cap: the path did not end
     }
-    atomicOr(&P.counters[CNT_ERR], 16u);  // bounce cap: the path did not end
+    warp_count(rays, &P.counters[CNT_RAYS]);
+    warp_count(shadows, &P.counters[CNT_SHRAYS]);
 }
 
 // ---------------------------------------------------------------- shadow rays
@@ -750,13 +774,16 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
 
 void launch_tail(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, const NrcCtx* nrc,
                  cudaStream_t st) {
-    const int blocks = (capacity + 127) / 128;
+    // n <= capacity paths, so many to a warp: at most capacity / 32 warps or the
+    // warps they spread over, and never more than paths
+    const uint32_t sms = (uint32_t)g_num_sms;
+    const int blocks = std::max((capacity + 127) / 128, std::min(g_num_sms * NR_TAIL_WARPS / 4, (capacity + 3) / 4));
     if (nrc) {
-        if (pol.trav) k_tail<true, true><<<blocks, 128, 0, st>>>(P, S, pol, *nrc);
-        else k_tail<true, false><<<blocks, 128, 0, st>>>(P, S, pol, *nrc);
+        if (pol.trav) k_tail<true, true><<<blocks, 128, 0, st>>>(P, S, pol, *nrc, sms);
+        else k_tail<true, false><<<blocks, 128, 0, st>>>(P, S, pol, *nrc, sms);
     } else {
-        if (pol.trav) k_tail<false, true><<<blocks, 128, 0, st>>>(P, S, pol, NrcCtx{});
-        else k_tail<false, false><<<blocks, 128, 0, st>>>(P, S, pol, NrcCtx{});
+        if (pol.trav) k_tail<false, true><<<blocks, 128, 0, st>>>(P, S, pol, NrcCtx{}, sms);
+        else k_tail<false, false><<<blocks, 128, 0, st>>>(P, S, pol, NrcCtx{}, sms);
     }
 }
 

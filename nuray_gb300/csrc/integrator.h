@@ -85,8 +85,8 @@ void launch_reset_counters(uint32_t* counters, cudaStream_t st);
 // that shade with kernels of their own (the adjoint replay).
 void launch_trace(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, cudaStream_t st);
 void launch_advance(uint32_t* counters, cudaStream_t st);
-// Every live path of queue_in to its end in one launch (after some
-// wavefront bounces of a small wave); capacity bounds the live count.
+// Every live path of queue_in to its end in one launch; capacity (> 0) bounds
+// the live count.
 void launch_tail(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, const NrcCtx* nrc,
                  cudaStream_t st);
 // k_trace's sort by shading category for hits recorded in P.hit by an earlier pass

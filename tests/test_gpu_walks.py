@@ -38,3 +38,26 @@ def test_small_trees_match_port(gpu_lib, port_lib, n, trav):
     d = np.stack([r.uniform(-0.5, 0.5, 500), r.uniform(-0.5, 0.5, 500), -np.ones(500)], 1).astype(np.float32)
     for a, b in zip(S.intersect(o, d, exhaustive=trav == 0), P.intersect(o, d)):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("policy", ["maxdepth=5 rrdepth=3", "prr=0.8", "maxdepth=1"])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (7, 5, 3), (97, 51, 4), (401, 303, 2), (640, 480, 5)])
+def test_automatic_tail_gives_the_wavefront_image(gpu_lib, w, h, spp, policy):
+    """By default one launch takes every path to its end from the bounce that
+    is known to start with few of them: the whole wave of the small frames
+    here (warps of 1 to 32 paths), some later bounce of the large one. The
+    light samples are rounded before they are added in both kernels, so the
+    image is that of tail=0 (the shading code inlined into the tail may
+    contract other multiply-adds: a few ulp). Both count every ray."""
+    from nuray_gb300 import scenes
+    sc = scenes.small_scene(9)
+    S = Scene.from_arrays(sc["pos"], sc["mat"], sc["mats"], uv=sc["uv"], nrm=sc["nrm"], textures=sc["textures"],
+                          env_tex=sc["env_tex"], env_gain=sc["env_gain"])
+    p = (f"renderer=ptnee imgw={w} imgh={h} spp={spp} campos=0,14,34 cameuler=0,-20,0 camfov=50 camasp={w / h:.4f} "
+         + policy)
+    a = S.render(p)
+    sa = S.stats()
+    b = S.render(p + " tail=0")
+    sb = S.stats()
+    np.testing.assert_allclose(a, b, rtol=1e-6, atol=1e-7)
+    assert (sa["rays"], sa["shadow_rays"]) == (sb["rays"], sb["shadow_rays"])
