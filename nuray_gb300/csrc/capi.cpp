@@ -272,6 +272,15 @@ void upload_scene(nr_scene* s) {
         if (!bad.empty()) throw NrError(NR_ERR_INVALID, bad);
     }
 
+    // each triangle's leaf, as the child it is
+    for (int k = 0; k < n; ++k) geo[3 * (size_t)k + 2].w = bits_f(-1);
+    for (int i = 0; i < ng; ++i)
+        for (int side = 0; side < 2; ++side) {
+            const int32_t r = side ? gn[i].d.y : gn[i].d.x;
+            if (r >= 0) continue;
+            for (int k = 0; k < nr::leaf_count(r); ++k) geo[3 * (size_t)(nr::leaf_first(r) + k) + 2].w = bits_f(2 * i + side);
+        }
+
     // The same nodes with every child box widened by delta for the one-FMA
     // box test without margin (fast_box). For a ray origin o with
     // |o_i| <= Bo and box bounds b with |b_i| <= A, the test's quotient

@@ -691,12 +691,17 @@ __global__ void k_nrc_targets(PathState P, NrcCtx C, float* __restrict__ y, floa
 }
 
 // ---------------------------------------------------------------- single queries
-__global__ void k_intersect(DeviceScene S, int n, const float* o, const float* d, int* tri, float* t, float* b1,
-                            float* b2, uint32_t* err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// One ray per lane, `take` rays per warp. MINB: minimum resident blocks per SM.
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) k_intersect(DeviceScene S, int n, int take, const float* __restrict__ o,
+                                                         const float* __restrict__ d, int* __restrict__ tri,
+                                                         float* __restrict__ t, float* __restrict__ b1,
+                                                         float* __restrict__ b2, uint32_t* err) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
+    if (lane >= take || i >= n) return;
     float tt, u, v;
-    int k = closest_hit(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
+    const int k = query_hit(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
     tri[i] = k >= 0 ? __float_as_int(__ldg(&S.tri_geo[3 * k]).w) : -1;
     t[i] = tt; b1[i] = u; b2[i] = v;
 }
@@ -825,9 +830,22 @@ void launch_finish(const float4* film, int npix, float inv_spp, float* hdr, uint
     k_finish<<<(npix + 255) / 256, 256, 0, st>>>(film, npix, inv_spp, hdr, rgb8);
 }
 
+// A call of few rays lasts as long as its slowest warp, and a warp as long as
+// its slowest ray in every phase: the rays are spread over the warps the chip
+// holds (40 per SM), one round of them up to 195k rays. Many rays want warps
+// in flight more than registers. us a call, 200k triangles, 4096 / 65,536
+// camera rays: 154 / 170 with closest_hit and full warps, 85 / 125 spread; 1M
+// triangles, 2 M rays off its surfaces in no order: 1387 with closest_hit,
+// 1063 / 1012 / 970 at 8 / 10 / 12 blocks per SM (60k rays: 132 / 121 / 137).
+// Measured and dropped: those rays sorted by origin and direction first, 923,
+// but 1100 against 271 where a million camera rays came in order already.
 void launch_intersect(const DeviceScene& S, int n, const float* o, const float* d, int* tri, float* t, float* b1,
                       float* b2, uint32_t* err, cudaStream_t st) {
-    k_intersect<<<(n + 127) / 128, 128, 0, st>>>(S, n, o, d, tri, t, b1, b2, err);
+    const int64_t warps = (int64_t)g_num_sms * 40;
+    const int take = (int)std::max<int64_t>(1, std::min<int64_t>(32, (n + warps - 1) / warps));
+    const unsigned blocks = (unsigned)(((int64_t)n + 4 * take - 1) / (4 * take));
+    if (n < (1 << 19)) k_intersect<10><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
+    else k_intersect<12><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
 }
 
 void launch_material_probe(const DeviceScene& S, int mat, int n, const float* wo, const float* nrm, const float* wi,

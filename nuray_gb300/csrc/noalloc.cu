@@ -13,6 +13,7 @@
 // does that, and looks up the array's address, when the first scene is
 // created on the device (noalloc_prepare), so the calls themselves load
 // and allocate nothing.
+#include <algorithm>
 #include <mutex>
 
 #include "nr_device.cuh"
@@ -44,13 +45,14 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 std::mutex g_mu;
 void* g_addr[NR_NOALLOC_MAX_DEVICES] = {};
 
-__global__ void k_intersect_noalloc(DeviceScene S, int n, const float* __restrict__ o, const float* __restrict__ d,
+__global__ void __launch_bounds__(128, 10) k_intersect_noalloc(DeviceScene S, int n, int take, const float* __restrict__ o, const float* __restrict__ d,
                                     int* __restrict__ tri, float* __restrict__ t, float* __restrict__ b1,
                                     float* __restrict__ b2, uint32_t* err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    // `take` rays per warp, as k_intersect
+    const int lane = threadIdx.x & 31, i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
+    if (lane >= take || i >= n) return;
     float tt, u, v;
-    int k = closest_hit(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
+    int k = query_hit(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
     tri[i] = k >= 0 ? __float_as_int(__ldg(&S.tri_geo[3 * k]).w) : -1;
     t[i] = tt;
     b1[i] = u;
@@ -107,7 +109,9 @@ std::string noalloc_intersect(const DeviceScene& S, int device, cudaStream_t st,
     if (e == cudaSuccess) e = cudaMemcpyAsync(so, o, f3, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(sd, d, f3, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return std::string("staging rays: ") + cudaGetErrorString(e);
-    k_intersect_noalloc<<<(n + 127) / 128, 128, 0, st>>>(S, n, so, sd, stri, stt, sb1, sb2, serr);
+    // rays spread over 40 warps on each of 152 SMs, as launch_intersect spreads them
+    const int take = std::max(1, std::min(32, (n + 152 * 40 - 1) / (152 * 40)));
+    k_intersect_noalloc<<<(n + 4 * take - 1) / (4 * take), 128, 0, st>>>(S, n, take, so, sd, stri, stt, sb1, sb2, serr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return std::string("k_intersect_noalloc: ") + cudaGetErrorString(e);
     uint32_t err = 0;

@@ -663,6 +663,95 @@ __device__ __forceinline__ int closest_hit_fast(const DeviceScene& S, f3 o, f3 d
     return best;
 }
 
+// closest_hit's answer by the widened boxes: its order (near first, a leaf at
+// once), its pruning, and its reach. A leaf the widened boxes reach counts
+// only if its exact box passes too, checked where one of its triangles is
+// hit: exact boxes nest and the exact quotients are monotone in the bounds, so
+// that is the reference's reach whatever stands above the leaf. For origins
+// within S.fast_origin_bound.
+__device__ __forceinline__ int closest_hit_query(const DeviceScene& S, f3 o, f3 d, float& best_t, float& best_b1,
+                                                 float& best_b2) {
+    best_t = 1e18f; best_b1 = 0.f; best_b2 = 0.f;
+    int best = -1, best_leaf = -1;
+    if (S.root_ref == INT32_MIN) return -1;
+    {
+        const SlabRay Q = make_slab_ray(o, d);
+        float te;
+        if (!box_test(Q, S.root_lo[0], S.root_hi[0], S.root_lo[1], S.root_hi[1], S.root_lo[2], S.root_hi[2], te)) return -1;
+    }
+    const FastRay R = make_fast_ray(make_slab_ray(o, d));
+    int2 stack[NR_STACK];
+    int sp = 0;
+    int ref = S.root_ref;
+    auto pop = [&]() {
+        while (sp > 0) {
+            const int2 e = stack[--sp];
+            if (__int_as_float(e.y) <= best_t * S.prune_k) return e.x;
+        }
+        return (int)NR_TRAV_END;
+    };
+    while (ref != NR_TRAV_END) {
+        while ((unsigned)ref < (unsigned)NR_TRAV_END) {
+            const FastNode& N = S.nodes_fast[ref];
+            const f8 a = ld8(N.c0), b = ld8(N.c1);
+            const float lim = fminf(best_t * S.prune_k, 1e18f);
+            float t0, t1;
+            const bool h0 = fast_box(R, a, lim, t0), h1 = fast_box(R, b, lim, t1);
+            const int k0 = __float_as_int(a.v[6]), k1 = __float_as_int(a.v[7]);
+            if (h0 && h1) {
+                int nr = k0, fr = k1;
+                float ft = t1;
+                if (t1 < t0) { nr = k1; fr = k0; ft = t0; }
+                stack[sp++] = make_int2(fr, __float_as_int(ft));
+                ref = nr;
+            } else if (h0) {
+                ref = k0;
+            } else if (h1) {
+                ref = k1;
+            } else {
+                ref = pop();
+            }
+        }
+        if (ref == NR_TRAV_END) break;
+        const int first = leaf_first(ref), cnt = leaf_count(ref);
+        float lt = 1e18f;
+        int li = -1;
+        for (int i = 0; i < cnt; ++i) {
+            const int ti = first + i;
+            const float4 g0 = __ldg(&S.tri_geo[3 * ti]), g1 = __ldg(&S.tri_geo[3 * ti + 1]), g2 = __ldg(&S.tri_geo[3 * ti + 2]);
+            float tt, u, v;
+            const float cap = fminf(lt, __uint_as_float(__float_as_uint(best_t) + 1u));
+            if (tri_test_fast(o, d, g0, g1, g2, cap, tt, u, v)) { lt = tt; li = ti; }
+        }
+        if (li >= 0 && (lt < best_t || (lt == best_t && first > best_leaf))) {
+            bool reached = true;
+            const int at = __float_as_int(__ldg(&S.tri_geo[3 * first + 2]).w);  // parent and side; -1: the root
+            if (at >= 0) {
+                const GpuNode& N = S.nodes[at >> 1];
+                const float4 xy = __ldg(at & 1 ? &N.b : &N.a), z = __ldg(&N.c);
+                float te;
+                reached = box_test(make_slab_ray(o, d), xy.x, xy.y, xy.z, xy.w, at & 1 ? z.z : z.x, at & 1 ? z.w : z.y, te) &&
+                          te <= best_t * S.prune_k;
+            }
+            if (reached) { best_t = lt; best = li; best_leaf = first; }
+        }
+        ref = pop();
+    }
+    if (best >= 0) {
+        const float4 g0 = __ldg(&S.tri_geo[3 * best]), g1 = __ldg(&S.tri_geo[3 * best + 1]), g2 = __ldg(&S.tri_geo[3 * best + 2]);
+        float t;
+        tri_test(o, d, g0, g1, g2, 3.0e38f, t, best_b1, best_b2);
+    }
+    return best;
+}
+
+// One ray of nr_intersect: closest_hit's answer, by the faster walk where it holds.
+__device__ __forceinline__ int query_hit(const DeviceScene& S, f3 o, f3 d, float& t, float& b1, float& b2, uint32_t* err) {
+    const float B = S.fast_origin_bound;
+    if (fabsf(o.x) <= B && fabsf(o.y) <= B && fabsf(o.z) <= B) return closest_hit_query(S, o, d, t, b1, b2);
+    return closest_hit(S, o, d, t, b1, b2, err);
+}
+
 // Any hit with t <= tmax on the widened boxes, as any_hit_ww. Child order
 // (1M-triangle frame, Mpaths/s): far first 759.8, near first 722.5.
 __device__ __forceinline__ bool any_hit_fast(const DeviceScene& S, f3 o, f3 d, float tmax,

@@ -45,8 +45,9 @@ struct alignas(64) FastNode {
 };
 
 // Per flattened triangle, traversal data, 48 bytes:
-//   g0 = (p0.xyz, loader index bits), g1 = (e1.xyz, material bits), g2 = (e2.xyz, 0)
+//   g0 = (p0.xyz, loader index bits), g1 = (e1.xyz, material bits), g2 = (e2.xyz, leaf bits)
 // with e1 = p1 - p0 and e2 = p2 - p0 rounded exactly as the reference does.
+// leaf bits: 2 x the inner node that holds the triangle's leaf as a child + which child; -1 where the root is the leaf.
 // Shading data, 64 bytes:
 //   s0 = (n0.xyz, t0.x), s1 = (n1.xyz, t0.y), s2 = (n2.xyz, t1.x), s3 = (t1.y, t2.x, t2.y, material bits)
 struct DeviceScene {

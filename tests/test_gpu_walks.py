@@ -61,3 +61,29 @@ def test_automatic_tail_gives_the_wavefront_image(gpu_lib, w, h, spp, policy):
     sb = S.stats()
     np.testing.assert_allclose(a, b, rtol=1e-6, atol=1e-7)
     assert (sa["rays"], sa["shadow_rays"]) == (sb["rays"], sb["shadow_rays"])
+
+
+@pytest.mark.parametrize("n", [1, 3, 31, 33, 6081, 65536, 65537, 194561, 524287, 524289])
+def test_query_spread_covers_every_ray(gpu_lib, port_lib, n):
+    """nr_intersect gives a warp 1 to 32 rays by their number, and another
+    build of its kernel from 2^19 on: every ray has its own answer, equal to
+    the restatement's on a sample, and the calls agree with each other."""
+    from nuray_gb300 import scenes
+    sc = scenes.small_scene(3, env=False, textures=False)
+    S, P = Scene.from_arrays(sc["pos"], sc["mat"], sc["mats"], uv=sc["uv"], nrm=sc["nrm"]), Oracle("port", sc)
+    r = np.random.default_rng(n)
+    lo, hi = sc["pos"].reshape(-1, 3).min(0), sc["pos"].reshape(-1, 3).max(0)
+    o = r.uniform(lo, hi, (n, 3)).astype(np.float32)
+    o[::5] = o[::5] * 40  # origins outside the widened boxes' bound take the exact walk
+    d = r.standard_normal((n, 3)).astype(np.float32)
+    got = S.intersect(o, d)
+    k = r.permutation(n)[:4000]
+    for a, b in zip((x[k] for x in got), P.intersect(o[k], d[k])):
+        assert np.mean(a == b) >= 0.999  # grazing rays may take another of two overlapping triangles
+    m = min(n, 65536)
+    from nuray_gb300._lib import check, lib
+    oc, dc = np.ascontiguousarray(o[:m]), np.ascontiguousarray(d[:m])
+    tri, t, b1, b2 = np.zeros(m, np.int32), *(np.zeros(m, np.float32) for _ in range(3))
+    check(lib().nr_intersect_noalloc(S._h, m, *(x.ctypes.data for x in (oc, dc, tri, t, b1, b2))))
+    for a, b in zip(got, (tri, t, b1, b2)):
+        np.testing.assert_array_equal(a[:m], b)
