@@ -145,7 +145,7 @@ struct nr_scene {
     nr::HostScene host;
     nr::Bvh bvh;
     nr::DeviceScene dev{};
-    DevBuf nodes, nodes_fast, tri_geo, tri_shade, mats, texels, tex_info, lights, light_cdf, light_guide, light_mat;
+    DevBuf nodes, wide, nodes_fast, tri_geo, tri_shade, mats, texels, tex_info, lights, light_cdf, light_guide, light_mat;
     DevBuf adj_L;  // per-path radiance for the adjoint replay
     DevBuf adj_wave;  // per-slot state of the wavefront adjoint replay
     DevBuf env_weight, env_row_cdf, env_col_cdf;  // environment sampling table (envis=1)
@@ -175,7 +175,7 @@ struct nr_scene {
         for (auto* b : all_bufs()) b->budget = &budget;
     }
     std::vector<DevBuf*> all_bufs() {
-        return {&nodes, &nodes_fast, &tri_geo, &tri_shade, &mats, &texels, &tex_info, &lights, &light_cdf, &light_guide,
+        return {&nodes, &wide, &nodes_fast, &tri_geo, &tri_shade, &mats, &texels, &tex_info, &lights, &light_cdf, &light_guide,
                 &light_mat,
                 &adj_L, &adj_wave, &env_weight, &env_row_cdf, &env_col_cdf, &path_mem, &film, &out_hdr, &out_rgb8,
                 &pix_list, &scratch, &nrc_mem};
@@ -197,7 +197,7 @@ namespace {
 
 uint64_t device_bytes(const nr_scene* s) {
     uint64_t b = 0;
-    for (auto* x : {&s->nodes, &s->nodes_fast, &s->tri_geo, &s->tri_shade, &s->mats, &s->texels, &s->tex_info, &s->lights,
+    for (auto* x : {&s->nodes, &s->wide, &s->nodes_fast, &s->tri_geo, &s->tri_shade, &s->mats, &s->texels, &s->tex_info, &s->lights,
                     &s->light_cdf, &s->light_guide, &s->light_mat})
         b += x->bytes;
     return b;
@@ -307,6 +307,26 @@ void upload_scene(nr_scene* s) {
                              {0, 0}};
     }
 
+    // The four-wide tree, as long as the walk's stack holds it (a tree of chains
+    // may need more than its depth: then two children per node) and 32-bit
+    // byte offsets reach it.
+    std::vector<nr::WideNodeHost> wide;
+    {
+        std::vector<int32_t> refs(2 * (size_t)ng);
+        std::vector<float> box(12 * (size_t)ng);
+        for (int i = 0; i < ng; ++i) {
+            const nr::GpuNode& g = gn[i];
+            refs[2 * (size_t)i] = g.d.x;
+            refs[2 * (size_t)i + 1] = g.d.y;
+            const float b[12] = {g.a.x, g.a.z, g.c.x, g.a.y, g.a.w, g.c.y, g.b.x, g.b.z, g.c.z, g.b.y, g.b.w, g.c.w};
+            std::copy(b, b + 12, &box[12 * (size_t)i]);
+        }
+        if (nr::build_wide(refs.data(), box.data(), ng, delta, 4, wide) > NR_STACK_LIMIT)
+            nr::build_wide(refs.data(), box.data(), ng, delta, 2, wide);
+        if (wide.size() >= (size_t(1) << 25)) wide.clear();
+    }
+    static_assert(sizeof(nr::WideNodeHost) == sizeof(nr::WideNode), "host and device node layouts");
+
     // emitters in loader order, weight = Triangle::area (twice the area)
     std::vector<float4> lt;
     std::vector<float> pdf;
@@ -367,6 +387,7 @@ void upload_scene(nr_scene* s) {
     upload(s->tri_shade, shade, st);
     upload(s->nodes, gn, st);
     upload(s->nodes_fast, gf, st);
+    upload(s->wide, wide, st);
     upload(s->mats, H.mats, st);
     upload(s->texels, texels, st);
     upload(s->tex_info, tinfo, st);
@@ -381,6 +402,7 @@ void upload_scene(nr_scene* s) {
 
     nr::DeviceScene& D = s->dev;
     D.nodes = s->nodes.as<nr::GpuNode>();
+    D.wide = s->wide.as<nr::WideNode>();  // null without nodes
     D.nodes_fast = s->nodes_fast.as<nr::FastNode>();
     D.fast_origin_bound = 2.0f * A + 4.0f * E;
     D.tri_geo = s->tri_geo.as<float4>();

@@ -775,4 +775,70 @@ std::string check_tree_refs(const int32_t* refs, int num_inner, int num_tris) {
     return "";
 }
 
+int build_wide(const int32_t* refs, const float* box, int num_inner, float delta, int width,
+               std::vector<WideNodeHost>& out) {
+    out.clear();
+    if (num_inner <= 0) return 0;
+    out.reserve((size_t)num_inner / 2 + 1);
+    struct Todo { int32_t node, parent, slot; };
+    std::vector<Todo> todo{{0, -1, 0}};
+    while (!todo.empty()) {
+        const Todo t = todo.back();
+        todo.pop_back();
+        const int32_t me = (int32_t)out.size();
+        if (t.parent >= 0) out[t.parent].ref[t.slot] = me;
+        // the children so far: binary references and where their boxes stand
+        int32_t ref[4];
+        const float* b[4];
+        int n = 2;
+        for (int k = 0; k < 2; ++k) {
+            ref[k] = refs[2 * (size_t)t.node + k];
+            b[k] = box + 12 * (size_t)t.node + 6 * k;
+        }
+        while (n < width) {
+            int open = -1;
+            float best = -1.f;
+            for (int k = 0; k < n; ++k) {
+                if (ref[k] < 0) continue;
+                const float x = b[k][3] - b[k][0], y = b[k][4] - b[k][1], z = b[k][5] - b[k][2];
+                const float area = x * y + y * z + z * x;
+                if (open < 0 || area > best) { open = k; best = area; }
+            }
+            if (open < 0) break;
+            const int32_t o = ref[open];
+            for (int k = n; k > open + 1; --k) { ref[k] = ref[k - 1]; b[k] = b[k - 1]; }
+            for (int k = 0; k < 2; ++k) {
+                ref[open + k] = refs[2 * (size_t)o + k];
+                b[open + k] = box + 12 * (size_t)o + 6 * k;
+            }
+            ++n;
+        }
+        WideNodeHost w;
+        for (int k = 0; k < 4; ++k) {
+            for (int a = 0; a < 3; ++a) {
+                w.plane[2 * a][k] = k < n ? b[k][a] - delta : INFINITY;
+                w.plane[2 * a + 1][k] = k < n ? b[k][3 + a] + delta : -INFINITY;
+            }
+            w.ref[k] = k < n ? ref[k] : -1;  // an empty leaf
+            w.pad[k] = 0;
+        }
+        out.push_back(w);
+        for (int k = n - 1; k >= 0; --k)  // the first child is taken next
+            if (ref[k] >= 0) todo.push_back({ref[k], me, k});
+    }
+    // children follow their parent: the stack each subtree needs, from the back
+    std::vector<int32_t> need(out.size(), 0);
+    for (size_t i = out.size(); i-- > 0;) {
+        int n = 0, deep = 0;
+        for (int k = 0; k < 4; ++k) {
+            const bool used = out[i].plane[0][k] <= out[i].plane[1][k] || out[i].ref[k] != -1;
+            if (!used) continue;
+            ++n;
+            if (out[i].ref[k] >= 0) deep = std::max(deep, (int)need[out[i].ref[k]]);
+        }
+        need[i] = n - 1 + deep;
+    }
+    return need[0];
+}
+
 }  // namespace nr

@@ -118,4 +118,22 @@ std::string bvh_from_arrays(const HostScene& s, int num_nodes, const float* box,
 // ends. Returns "" or what is wrong.
 std::string check_tree_refs(const int32_t* refs, int num_inner, int num_tris);
 
+// A node of the four-wide tree as the device reads it (WideNode,
+// nr_types.h): plane[2 a] the lower and plane[2 a + 1] the upper bounds of
+// the four children along axis a.
+struct WideNodeHost {
+    float plane[6][4];
+    int32_t ref[4];
+    int32_t pad[4];
+};
+// Collapses the binary tree (inner nodes in depth-first order, children as in
+// check_tree_refs' references, box[12] per inner node: left min, max, right
+// min, max) into nodes of up to `width` (2 to 4) children: a node starts with
+// its two children and opens the inner child of the largest surface until it
+// has `width`. Every box grows by delta on each side. Nodes come depth-first,
+// a parent before its children. Returns the deepest stack a depth-first walk
+// that pushes all hit children but one needs.
+int build_wide(const int32_t* refs, const float* box, int num_inner, float delta, int width,
+               std::vector<WideNodeHost>& out);
+
 }  // namespace nr

@@ -234,8 +234,8 @@ __device__ __forceinline__ bool nrc_is_training(uint32_t pixel, uint32_t sample,
 // Queues a shadow ray (or, when no hit can come before the limit, adds its
 // contribution at once). rec: the training record whose target leaves this
 // light sample out, or -1.
-// TAIL: trace the shadow ray here (1: exact walk, 2: fast) instead of
-// queueing it. env: the vertex's environment sample, queued with its limit
+// TAIL: trace the shadow ray here (1: exact walk, 2: fast, 3: four-wide)
+// instead of queueing it. env: the vertex's environment sample, queued with its limit
 // negated: k_shadow leaves its contribution in the queue entry (zero when
 // occluded) and k_env_fold adds it after the area-light samples, so each
 // path's radiance has one writer at a time and the restatement's order.
@@ -245,8 +245,9 @@ __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScen
                                             uint32_t* shadows, bool env = false) {
     if (TAIL && tmax > 0.f) {
         ++*shadows;
-        const bool occluded = TAIL == 2 ? any_hit_fast(S, so, d, tmax)
-                                        : any_hit_ww<false>(S, so, d, tmax, &P.counters[CNT_ERR]);
+        const bool occluded = TAIL == 3   ? any_hit_wide(S, so, d, tmax)
+                              : TAIL == 2 ? any_hit_fast(S, so, d, tmax)
+                                          : any_hit_ww<false>(S, so, d, tmax, &P.counters[CNT_ERR]);
         if (occluded) return;
         tmax = 0.f;  // unoccluded: added below
     }
@@ -270,8 +271,8 @@ __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScen
 
 // MT: the shading category when it is known at compile time (a material
 // type, or CAT_MISS), -1 for any. TAIL: light samples traced here (1 by the
-// exact walk, 2 by the fast one) and the continuing path not queued. Returns
-// whether the path goes on.
+// exact walk, 2 by the fast, 3 by the four-wide one) and the continuing path
+// not queued. Returns whether the path goes on.
 template <bool NRC, int MT = -1, int TAIL = 0>
 __device__ __forceinline__ bool shade_one(const PathState& P, const DeviceScene& S, const Policy& pol, int slot,
                                           const NrcCtx& C, uint32_t* shadows = nullptr) {
@@ -520,6 +521,10 @@ static void launch_shade(const PathState& P, const DeviceScene& S, const Policy&
 #ifndef NR_TAIL_MINB
 #define NR_TAIL_MINB 8
 #endif
+// With the four-wide walk (few paths) the registers pay more: 3072 paths 181
+// us at 8 blocks, 178 at 6; 57,600 365 / 354; 522,240 of every material (about
+// half of them live at the tail) 730 / 716.
+#define NR_TAIL_MINB_WIDE 6
 // Paths of a warp: a warp walks for as long as its slowest ray in every
 // phase, so a few paths are spread over 16 warps per SM, and up to 8 warps
 // per SM before warps fill (the whole path in this kernel, 1M triangles, 3072
@@ -532,8 +537,9 @@ __host__ __device__ inline uint32_t tail_paths_per_warp(uint32_t n, uint32_t sms
     const uint32_t take = (n + warps - 1u) / warps;
     return take < 1u ? 1u : (take > 32u ? 32u : take);
 }
-template <bool NRC, bool FAST>
-__global__ void __launch_bounds__(128, NR_TAIL_MINB) k_tail(PathState P, DeviceScene S, Policy pol, NrcCtx C,
+// WALK: 1 exact, 2 fast, 3 four-wide.
+template <bool NRC, int WALK>
+__global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_MINB) k_tail(PathState P, DeviceScene S, Policy pol, NrcCtx C,
                                                               uint32_t sms) {
     const uint32_t n = P.counters[CNT_IN], take = tail_paths_per_warp(n, sms);
     const uint32_t lane = threadIdx.x & 31u, i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
@@ -544,10 +550,12 @@ __global__ void __launch_bounds__(128, NR_TAIL_MINB) k_tail(PathState P, DeviceS
         for (int b = 0; on && b < NR_TAIL_MAX_BOUNCES; ++b) {
             const f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
             float t, b1, b2;
-            const int tri = FAST ? closest_hit_fast(S, o, d, t, b1, b2) : closest_hit_ww(S, o, d, t, b1, b2);
+            const int tri = WALK == 3   ? closest_hit_wide<false>(S, o, d, t, b1, b2)
+                            : WALK == 2 ? closest_hit_fast(S, o, d, t, b1, b2)
+                                        : closest_hit_ww(S, o, d, t, b1, b2);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
             ++rays;
-            on = shade_one<NRC, -1, FAST ? 2 : 1>(P, S, pol, slot, C, &shadows);
+            on = shade_one<NRC, -1, WALK>(P, S, pol, slot, C, &shadows);
         }
         if (on) atomicOr(&P.counters[CNT_ERR], (uint32_t)NR_ERRBIT_BOUNCES);  // bounce cap: the path did not end
     }
@@ -691,8 +699,9 @@ __global__ void k_nrc_targets(PathState P, NrcCtx C, float* __restrict__ y, floa
 }
 
 // ---------------------------------------------------------------- single queries
-// One ray per lane, `take` rays per warp. MINB: minimum resident blocks per SM.
-template <int MINB>
+// One ray per lane, `take` rays per warp. MINB: minimum resident blocks per
+// SM; WIDE: the four-wide walk.
+template <int MINB, bool WIDE>
 __global__ void __launch_bounds__(128, MINB) k_intersect(DeviceScene S, int n, int take, const float* __restrict__ o,
                                                          const float* __restrict__ d, int* __restrict__ tri,
                                                          float* __restrict__ t, float* __restrict__ b1,
@@ -701,7 +710,7 @@ __global__ void __launch_bounds__(128, MINB) k_intersect(DeviceScene S, int n, i
     const int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
     if (lane >= take || i >= n) return;
     float tt, u, v;
-    const int k = query_hit(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
+    const int k = query_hit<WIDE>(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
     tri[i] = k >= 0 ? __float_as_int(__ldg(&S.tri_geo[3 * k]).w) : -1;
     t[i] = tt; b1[i] = u; b2[i] = v;
 }
@@ -783,12 +792,16 @@ void launch_tail(const PathState& P, const DeviceScene& S, const Policy& pol, in
     // warps they spread over, and never more than paths
     const uint32_t sms = (uint32_t)g_num_sms;
     const int blocks = std::max((capacity + 127) / 128, std::min(g_num_sms * NR_TAIL_WARPS / 4, (capacity + 3) / 4));
-    if (nrc) {
-        if (pol.trav) k_tail<true, true><<<blocks, 128, 0, st>>>(P, S, pol, *nrc, sms);
-        else k_tail<true, false><<<blocks, 128, 0, st>>>(P, S, pol, *nrc, sms);
-    } else {
-        if (pol.trav) k_tail<false, true><<<blocks, 128, 0, st>>>(P, S, pol, NrcCtx{}, sms);
-        else k_tail<false, false><<<blocks, 128, 0, st>>>(P, S, pol, NrcCtx{}, sms);
+    // the four-wide walk up to the count where it stops paying
+    const int walk = pol.trav == 0 ? 1 : (S.wide && capacity <= 300000 ? 3 : 2);
+    const NrcCtx C = nrc ? *nrc : NrcCtx{};
+    switch (walk + (nrc ? 3 : 0)) {
+        case 1: k_tail<false, 1><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
+        case 2: k_tail<false, 2><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
+        case 3: k_tail<false, 3><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
+        case 4: k_tail<true, 1><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
+        case 5: k_tail<true, 2><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
+        default: k_tail<true, 3><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
     }
 }
 
@@ -832,20 +845,22 @@ void launch_finish(const float4* film, int npix, float inv_spp, float* hdr, uint
 
 // A call of few rays lasts as long as its slowest warp, and a warp as long as
 // its slowest ray in every phase: the rays are spread over the warps the chip
-// holds (40 per SM), one round of them up to 195k rays. Many rays want warps
-// in flight more than registers. us a call, 200k triangles, 4096 / 65,536
-// camera rays: 154 / 170 with closest_hit and full warps, 85 / 125 spread; 1M
-// triangles, 2 M rays off its surfaces in no order: 1387 with closest_hit,
-// 1063 / 1012 / 970 at 8 / 10 / 12 blocks per SM (60k rays: 132 / 121 / 137).
-// Measured and dropped: those rays sorted by origin and direction first, 923,
-// but 1100 against 271 where a million camera rays came in order already.
+// holds (32 per SM), one round of them up to 156k rays, and take the four-wide
+// walk. Many rays want warps in flight more than registers or short walks. us
+// a call, 200k triangles, 4096 / 65,536 / 262,144 camera rays: 154 / 170 / 205
+// with closest_hit and full warps, 85 / 125 / 172 with closest_hit_query
+// spread, 71 / 108 / 140 four-wide; 1M triangles, 2 M rays off its surfaces in
+// no order: 1387 with closest_hit, 1063 / 1012 / 970 with closest_hit_query at
+// 8 / 10 / 12 blocks per SM. Measured and dropped: those rays sorted by origin
+// and direction first, 923, but 1100 against 271 where a million camera rays
+// came in order already.
 void launch_intersect(const DeviceScene& S, int n, const float* o, const float* d, int* tri, float* t, float* b1,
                       float* b2, uint32_t* err, cudaStream_t st) {
-    const int64_t warps = (int64_t)g_num_sms * 40;
+    const int64_t warps = (int64_t)g_num_sms * 32;
     const int take = (int)std::max<int64_t>(1, std::min<int64_t>(32, (n + warps - 1) / warps));
     const unsigned blocks = (unsigned)(((int64_t)n + 4 * take - 1) / (4 * take));
-    if (n < (1 << 19)) k_intersect<10><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
-    else k_intersect<12><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
+    if (n < (1 << 19) && S.wide) k_intersect<8, true><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
+    else k_intersect<12, false><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
 }
 
 void launch_material_probe(const DeviceScene& S, int mat, int n, const float* wo, const float* nrm, const float* wi,

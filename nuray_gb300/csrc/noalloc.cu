@@ -45,14 +45,15 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 std::mutex g_mu;
 void* g_addr[NR_NOALLOC_MAX_DEVICES] = {};
 
-__global__ void __launch_bounds__(128, 10) k_intersect_noalloc(DeviceScene S, int n, int take, const float* __restrict__ o, const float* __restrict__ d,
+template <bool WIDE>
+__global__ void __launch_bounds__(128, 8) k_intersect_noalloc(DeviceScene S, int n, int take, const float* __restrict__ o, const float* __restrict__ d,
                                     int* __restrict__ tri, float* __restrict__ t, float* __restrict__ b1,
                                     float* __restrict__ b2, uint32_t* err) {
     // `take` rays per warp, as k_intersect
     const int lane = threadIdx.x & 31, i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
     if (lane >= take || i >= n) return;
     float tt, u, v;
-    int k = query_hit(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
+    int k = query_hit<WIDE>(S, mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2]), tt, u, v, err);
     tri[i] = k >= 0 ? __float_as_int(__ldg(&S.tri_geo[3 * k]).w) : -1;
     t[i] = tt;
     b1[i] = u;
@@ -109,9 +110,10 @@ std::string noalloc_intersect(const DeviceScene& S, int device, cudaStream_t st,
     if (e == cudaSuccess) e = cudaMemcpyAsync(so, o, f3, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(sd, d, f3, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return std::string("staging rays: ") + cudaGetErrorString(e);
-    // rays spread over 40 warps on each of 152 SMs, as launch_intersect spreads them
-    const int take = std::max(1, std::min(32, (n + 152 * 40 - 1) / (152 * 40)));
-    k_intersect_noalloc<<<(n + 4 * take - 1) / (4 * take), 128, 0, st>>>(S, n, take, so, sd, stri, stt, sb1, sb2, serr);
+    // rays spread over 32 warps on each of 152 SMs, as launch_intersect spreads them
+    const int take = std::max(1, std::min(32, (n + 152 * 32 - 1) / (152 * 32))), blocks = (n + 4 * take - 1) / (4 * take);
+    if (S.wide) k_intersect_noalloc<true><<<blocks, 128, 0, st>>>(S, n, take, so, sd, stri, stt, sb1, sb2, serr);
+    else k_intersect_noalloc<false><<<blocks, 128, 0, st>>>(S, n, take, so, sd, stri, stt, sb1, sb2, serr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return std::string("k_intersect_noalloc: ") + cudaGetErrorString(e);
     uint32_t err = 0;

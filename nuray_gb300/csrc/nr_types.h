@@ -44,6 +44,18 @@ struct alignas(64) FastNode {
     int32_t pad[2];
 };
 
+// Four-wide node for walks of few rays, 128 bytes (one cache line): the boxes
+// of up to four children by coordinate, so that a ray picks the near and far
+// planes of an axis by address from its direction's sign, then the child
+// references (inner nodes as indices into the wide array). Boxes are widened as
+// FastNode's. Unused children have an empty box and an empty leaf. Host
+// counterpart: WideNodeHost (host_scene.h).
+struct alignas(128) WideNode {
+    float4 plane[6];  // lo.x, hi.x, lo.y, hi.y, lo.z, hi.z of the four children
+    int4 ref;
+    int4 pad;
+};
+
 // Per flattened triangle, traversal data, 48 bytes:
 //   g0 = (p0.xyz, loader index bits), g1 = (e1.xyz, material bits), g2 = (e2.xyz, leaf bits)
 // with e1 = p1 - p0 and e2 = p2 - p0 rounded exactly as the reference does.
@@ -79,6 +91,7 @@ struct DeviceScene {
     int32_t num_nodes;        // internal nodes
     float prune_k;            // subtrees entered beyond prune_k x the best hit are skipped (infinity: none)
     const FastNode* nodes_fast;  // the same nodes with every box widened, for the fast walk (trav=1)
+    const WideNode* wide;        // the four-wide tree, or null (a scene of one leaf, or more than 2^25 nodes)
     float fast_origin_bound;     // the fast walk is conservative for ray origins with every |coordinate| <= this
 };
 
