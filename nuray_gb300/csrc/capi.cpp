@@ -1263,8 +1263,16 @@ int nr_scene_set_materials(nr_scene* s, int32_t n, const nr_material* mats) {
         std::lock_guard<std::mutex> lk(s->mu);
         NR_CUDA(cudaSetDevice(s->device));
         s->host.mats.assign(mats, mats + n);
-        // emitter colours live in the emitter table as well: rebuild it with the materials
-        upload_scene(s);
+        // On the device the materials stand in one table, and the emitters'
+        // radiance in the light table as well; types, and with them everything
+        // else the scene derives, are the same. (Rebuilding and uploading the
+        // scene instead: 6.7 ms for 200k triangles, against 0.03 ms.)
+        NR_CUDA(cudaMemcpyAsync(s->mats.p, s->host.mats.data(), s->host.mats.size() * sizeof(nr_material), cudaMemcpyHostToDevice,
+                                s->stream));
+        nr::launch_set_emission(s->lights.as<float4>(), s->light_mat.as<int32_t>(), s->mats.as<nr_material>(), s->dev.num_lights,
+                                s->stream);
+        NR_CUDA(cudaGetLastError());
+        NR_CUDA(cudaStreamSynchronize(s->stream));
     });
 }
 

@@ -715,6 +715,16 @@ __global__ void __launch_bounds__(128, MINB) k_intersect(DeviceScene S, int n, i
     t[i] = tt; b1[i] = u; b2[i] = v;
 }
 
+// The emitters' radiance from their materials (the light table's layout,
+// upload_scene).
+__global__ void k_set_emission(float4* __restrict__ lights, const int32_t* __restrict__ light_mat,
+                               const nr_material* __restrict__ mats, int num_lights) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= num_lights) return;
+    const nr_material& M = mats[light_mat[i]];
+    for (int k = 0; k < 3; ++k) lights[6 * (size_t)i + k].w = M.c0[k];
+}
+
 struct ListRng {
     const float* u;
     int i;
@@ -861,6 +871,10 @@ void launch_intersect(const DeviceScene& S, int n, const float* o, const float* 
     const unsigned blocks = (unsigned)(((int64_t)n + 4 * take - 1) / (4 * take));
     if (n < (1 << 19) && S.wide) k_intersect<8, true><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
     else k_intersect<12, false><<<blocks, 128, 0, st>>>(S, n, take, o, d, tri, t, b1, b2, err);
+}
+
+void launch_set_emission(float4* lights, const int32_t* light_mat, const nr_material* mats, int num_lights, cudaStream_t st) {
+    if (num_lights > 0) k_set_emission<<<(num_lights + 127) / 128, 128, 0, st>>>(lights, light_mat, mats, num_lights);
 }
 
 void launch_material_probe(const DeviceScene& S, int mat, int n, const float* wo, const float* nrm, const float* wi,

@@ -97,6 +97,8 @@ void launch_collect(const PathState& P, const WaveDesc& W, float* out, int spp, 
 void launch_finish(const float4* film, int npix, float inv_spp, float* hdr, uint8_t* rgb8, cudaStream_t st);
 void launch_intersect(const DeviceScene& S, int n, const float* o, const float* d, int* tri, float* t, float* b1,
                       float* b2, uint32_t* err, cudaStream_t st);
+// Rewrites the emitters' radiance in the light table from their materials.
+void launch_set_emission(float4* lights, const int32_t* light_mat, const nr_material* mats, int num_lights, cudaStream_t st);
 void launch_material_probe(const DeviceScene& S, int mat, int n, const float* wo, const float* nrm, const float* wi,
                            const float* uv, const float* u, float* f, float* pdf, float* wi_s, cudaStream_t st);
 
