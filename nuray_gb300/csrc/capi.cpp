@@ -60,9 +60,11 @@ int guarded(F&& f) {
 // Device bytes a scene may hold (scene option max_device_bytes): every
 // buffer of the scene draws on it, and an allocation past it fails with
 // NR_ERR_OOM as a failed cudaMalloc does.
+struct DevBuf;
 struct Budget {
     size_t cap = SIZE_MAX;
     size_t used = 0;
+    DevBuf* spare = nullptr;  // a buffer its user can do without: given up where another does not fit
 };
 
 struct DevBuf {
@@ -73,15 +75,26 @@ struct DevBuf {
     // touching the old buffer; if cudaMalloc fails the buffer is left empty,
     // so callers that cache sizes or pointers into it reset them first.
     void alloc(size_t n) {
-        if (budget && n > budget->cap - (budget->used - bytes))
+        if (budget && n > budget->cap - (budget->used - bytes) && !(drop_spare() && n <= budget->cap - (budget->used - bytes)))
             throw NrError(NR_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes exceeds the scene's cap of " +
                                           std::to_string(budget->cap) + " bytes (" +
                                           std::to_string(budget->used - bytes) + " in use)");
         release();
         if (n == 0) return;
-        NR_CUDA(cudaMalloc(&p, n));
+        cudaError_t e = cudaMalloc(&p, n);
+        if (e == cudaErrorMemoryAllocation && drop_spare()) {
+            (void)cudaGetLastError();
+            e = cudaMalloc(&p, n);
+        }
+        if (e != cudaSuccess) p = nullptr;
+        NR_CUDA(e);
         bytes = n;
         if (budget) budget->used += n;
+    }
+    bool drop_spare() {
+        if (!budget || !budget->spare || budget->spare == this || !budget->spare->p) return false;
+        budget->spare->release();  // cudaFree waits for the device
+        return true;
     }
     void release() {
         if (p) cudaFree(p);
@@ -151,7 +164,7 @@ struct nr_scene {
     DevBuf env_weight, env_row_cdf, env_col_cdf;  // environment sampling table (envis=1)
     int num_gpu_nodes = 0;
     // wavefront state
-    DevBuf path_mem, film, out_hdr, out_rgb8, pix_list, scratch;
+    DevBuf path_mem, sort_mem, film, out_hdr, out_rgb8, pix_list, scratch;
     int film_pixels = 0;
     uint64_t film_samples = 0;  // samples summed in film (accumulate=1 keeps adding)
     nr::PathState ps{};
@@ -173,11 +186,12 @@ struct nr_scene {
 
     nr_scene() {
         for (auto* b : all_bufs()) b->budget = &budget;
+        budget.spare = &sort_mem;
     }
     std::vector<DevBuf*> all_bufs() {
         return {&nodes, &wide, &nodes_fast, &tri_geo, &tri_shade, &mats, &texels, &tex_info, &lights, &light_cdf, &light_guide,
                 &light_mat,
-                &adj_L, &adj_wave, &env_weight, &env_row_cdf, &env_col_cdf, &path_mem, &film, &out_hdr, &out_rgb8,
+                &adj_L, &adj_wave, &env_weight, &env_row_cdf, &env_col_cdf, &path_mem, &sort_mem, &film, &out_hdr, &out_rgb8,
                 &pix_list, &scratch, &nrc_mem};
     }
 
@@ -490,7 +504,7 @@ void finish_scene(nr_scene* s, const char* options, nr::Bvh* prebuilt = nullptr)
 // call needs to start from.
 void release_work_buffers(nr_scene* s) {
     cudaStreamSynchronize(s->stream);
-    for (auto* b : {&s->path_mem, &s->film, &s->out_hdr, &s->out_rgb8, &s->pix_list, &s->scratch, &s->adj_L,
+    for (auto* b : {&s->path_mem, &s->sort_mem, &s->film, &s->out_hdr, &s->out_rgb8, &s->pix_list, &s->scratch, &s->adj_L,
                     &s->adj_wave, &s->nrc_mem})
         b->release();
     s->capacity = 0;
@@ -552,6 +566,46 @@ void ensure_paths(nr_scene* s, int cap, int sh_mult = 1) {
     NR_CUDA(cudaMemsetAsync(P.counters, 0, nr::NUM_COUNTERS * 4, s->stream));
     s->capacity = cap;
     s->sh_mult = sh_mult;
+}
+
+// The ray sort's workspace for a bounce of `live` paths in waves of cap, into
+// P; P.sort.place stays null where the rays are not sorted. They are in
+// scenes whose tree outgrows an SM's L1, and bounces of 4M paths or more: a
+// sort costs some 0.1 ms and 60 ps a ray. ms without / with it, 1M triangles:
+// 132.7M paths 140.1 / 120.9, 33.2M 36.4 / 32.2, 8.3M 10.3 / 9.7, 4.1M 5.78 /
+// 5.62 (sorting bounces from 1M paths on 5.73, from 0.2M on 5.73; 2.1M paths
+// from 1M on 3.44 / 3.52); 200k triangles, 8.4M 7.59 / 7.02; sky with its
+// samples, 8.3M 13.4 / 12.7; 1720 triangles, 8.4M 3.89 / 3.88; 36 triangles, 4.9M
+// 5.53 / 5.49. Bits an axis of the origin and of the direction: 132.7M paths
+// 4+3 130.0, 5+3 124.7, 6+2 124.5, 6+3 120.9; 8.3M 4+3 9.90, 5+3 9.67, 6+3 9.81.
+// Without room for the workspace the rays stay in queue order.
+void ensure_sort(nr_scene* s, int cap, int live, int sh_mult, nr::PathState& P) {
+    nr::RaySort& R = P.sort;
+    R.input = R.place[0] ? 1 : 0;  // what the bounce before did
+    R.place[0] = R.place[1] = nullptr;
+    if (live < 4000000 || s->dev.num_tris < 16384) return;
+    R.origin_bits = cap >= (1 << 24) && s->dev.num_tris >= (1 << 19) ? 6 : 5;
+    R.dir_bits = 3;
+    float ext = 0.f;
+    for (int k = 0; k < 3; ++k) ext = std::max(ext, s->dev.root_hi[k] - s->dev.root_lo[k]);
+    R.cells_per_unit = ext > 0.f ? (float)(1 << R.origin_bits) / ext : 0.f;
+    const size_t C = (size_t)cap, CS = C * (size_t)sh_mult, nb = R.buckets();
+    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+    try {
+        s->sort_mem.ensure(al(CS * 8) + al(C * 8) + 2 * al(nb * 4) + 2 * al(nb / 4096 * 4) + al(CS * 4) + al(C * 4));
+    } catch (const NrError& e) {
+        if (e.code != NR_ERR_OOM) throw;
+        (void)cudaGetLastError();
+        return;
+    }
+    char* p = s->sort_mem.as<char>();
+    auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
+    R.place[0] = (uint2*)take(CS * 8);
+    R.place[1] = (uint2*)take(C * 8);
+    for (auto& h : R.hist) h = (uint32_t*)take(nb * 4);
+    for (auto& h : R.part) h = (uint32_t*)take(nb / 4096 * 4);
+    R.order = (int32_t*)take(CS * 4);
+    R.queue = (int32_t*)take(C * 4);
 }
 
 // Sizes the batch scratch of a cache for m rows.
@@ -801,17 +855,21 @@ void wave_layout(const RenderArgs& A, bool has_pix_list, nr::WaveDesc& W) {
 // NR_TAIL_MAX_BOUNCES too): paths end by Russian roulette, misses and
 // emitters, but prr = 1 in a closed scene would never end.
 constexpr int kMaxBounces = 4096;
-// Paths entering a bounce at or below which the tail kernel takes them all to
-// their end. Its warps shade whatever material each lane met, so the line
-// lies lower where several surface types occur, and lower still for a whole
-// wave, whose bounces mostly lie ahead. ms with the line below / above the
-// count, 1M triangles of one type: 230k paths 1.12 / 0.77, 518k 1.55 / 1.35,
-// 1.04M 2.12 / 2.35; every type, unbounded paths: 246k 0.64 / 0.60, 522k 0.76 /
-// 0.97; a room of four types: 246k 0.94 / 1.26, 1.04M with 1.75 from 150k on,
-// 2.52 from 600k on; sky and dielectrics, 518k 1.70 / 2.02.
+// Paths known to enter a bounce (the count of the one before it, from bounce 2
+// on) at or below which the tail kernel takes them all to their end. Its warps
+// shade whatever material each lane met, so the line lies lower where several
+// surface types occur, and lower still for a whole wave, whose bounces mostly
+// lie ahead. ms of the whole wave in the tail / two wavefront bounces first, 1M
+// triangles of one type: 261k paths 0.84 / 0.99, 518k 1.35 / 1.41, 1.04M 2.35 /
+// 2.10; sky and dielectrics: 61k 0.76 / 0.95, 123k 1.10 / 1.15, 184k 1.68 /
+// 1.34; every type: 61k 0.30 / 0.37, 184k 0.51 / 0.49; a room of four types:
+// 61k 0.30 / 0.34, 123k 0.51 / 0.45, 261k 1.01 / 0.81. Later bounces, the room,
+// 1.04M unbounded paths: 1.81 / 1.75 / 1.92 / 2.52 with the line at 50k / 150k /
+// 300k / 600k; every type, 522k: 0.86 / 0.84 / 0.77 / 0.97.
 int64_t tail_limit(uint32_t cat_mask, int bounce) {
     const int surfaces = __builtin_popcount(cat_mask & ((1u << NR_MAT_LIGHT) - 1u));
-    return surfaces <= 1 ? 600000 : (bounce == 0 ? 200000 : 300000);
+    if (surfaces <= 1) return 600000;
+    return bounce == 0 ? 100000 : (bounce == 1 ? 0 : 300000);
 }
 
 void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pix, int sample0, float4* film,
@@ -940,12 +998,14 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
                 ev_kind.push_back(-1); ev_kind.push_back(0); ev_kind.push_back(1); ev_kind.push_back(2);
                 nev += 4;
             }
+            ensure_sort(s, cap, live, s->sh_mult, P);
             nr::launch_bounce(P, D, A.pol, cap, live, st, A.profile ? evs : nullptr, A.count,
                               use_nrc ? &s->nrc_ctx : nullptr);
             std::swap(P.queue_in, P.queue_out);
             S.bounces++;
             S.trace_launches++;
-            S.kernel_launches += nr::bounce_launches(cap, A.pol.envis != 0, s->dev.cat_mask);
+            S.kernel_launches += nr::bounce_launches(cap, A.pol.envis != 0, s->dev.cat_mask) +
+                                 (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
             // The count entering the next bounce, read back; the one asked for
             // a bounce earlier is taken now, while this bounce runs.
             const bool last = A.pol.maxdepth > 0 && bounce + 1 >= A.pol.maxdepth;
@@ -1106,9 +1166,10 @@ uint64_t adjoint_waves(nr_scene* s, const RenderArgs& A, int npix, const float* 
             const bool rec = bounce < depth_rec;
             P.hit = rec ? rec_hit + (size_t)bounce * C : s->ps.hit;
             P.vis = rec ? rec_vis + (size_t)bounce * C : nullptr;
+            ensure_sort(s, cap, live, s->sh_mult, P);
             nr::launch_bounce(P, D, pol1, cap, live, st, nullptr, false, nullptr);
             std::swap(P.queue_in, P.queue_out);
-            launches += nr::bounce_launches(cap, false, s->dev.cat_mask);
+            launches += nr::bounce_launches(cap, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
             if (!live_after(bounce, live)) break;
         }
         nr::launch_collect(s->ps, W, s->adj_L.as<float>(), A.spp, A.pol.imgw, st);

@@ -12,6 +12,7 @@
 
 #include "nr_material.cuh"
 #include "integrator.h"
+#include "ray_sort.cuh"
 
 namespace nr {
 
@@ -88,8 +89,8 @@ __device__ __forceinline__ void warp_count(uint32_t v, uint32_t* lohi) {
 // Closest hit, persistent: warps take 32 queue entries at a time from a
 // shared cursor, one ray per lane to completion, then the slot is bucketed by
 // shading category (material type of the hit, or CAT_MISS).
-// FAST (trav=1) walks the widened boxes (closest_hit_fast); !FAST (trav=0)
-// the reference's boxes with its exact arithmetic (closest_hit_ww). The
+// trav=1 walks the widened boxes (closest_hit_fast), trav=0 the reference's
+// boxes with its exact arithmetic (closest_hit_ww). The
 // widened boxes accept every box the exact test accepts, so trav=1 reaches
 // every triangle trav=0 reaches (the same hits but where a ray passes within
 // about 1e-6 of a box face and hits a triangle there that the exact test's
@@ -114,7 +115,8 @@ __device__ __forceinline__ void warp_count(uint32_t v, uint32_t* lohi) {
 #ifndef NR_SHADOW_MINB
 #define NR_SHADOW_MINB 10
 #endif
-template <bool COUNT, bool FAST>
+// WALK: 0 exact; 1 fast, leaves postponed; 2 fast, for a sorted queue.
+template <bool COUNT, int WALK>
 __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, DeviceScene S, int capacity) {
     const uint32_t n = P.counters[CNT_IN];
     const int lane = threadIdx.x & 31;
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, Devic
             int slot = P.queue_in[idx];
             f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
             float t, b1, b2;
-            const int tri = FAST ? closest_hit_fast(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr)
+            const int tri = WALK ? closest_hit_fast<WALK == 1>(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr)
                                  : closest_hit_ww(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
             int cat = CAT_MISS;
@@ -162,6 +164,7 @@ __global__ void k_sort_recorded(PathState P, DeviceScene S, int capacity) {
 // has t <= the ray's limit (any_hit); unoccluded rays add their NEE term.
 template <bool COUNT, bool FAST>
 __global__ void __launch_bounds__(128, NR_SHADOW_MINB) k_shadow(PathState P, DeviceScene S, float4* t_before) {
+    const int32_t* __restrict__ order = P.sort.place[0] ? P.sort.order : nullptr;  // of a sorted queue
     // (a full queue drops rays with an error bit but still counts them)
     const uint32_t n = min(P.counters[CNT_SHADOW], (uint32_t)P.sh_cap);
     const int lane = threadIdx.x & 31;
@@ -173,6 +176,7 @@ __global__ void __launch_bounds__(128, NR_SHADOW_MINB) k_shadow(PathState P, Dev
         if (base >= n) break;
         uint32_t idx = base + lane;
         if (idx < n) {
+            if (order) idx = (uint32_t)order[idx];
             float4 o = P.sh_o[idx], d = P.sh_d[idx];
             const bool env = o.w < 0.f;  // an environment sample: k_env_fold adds it
             const float tmax = env ? -o.w : o.w;
@@ -257,6 +261,7 @@ __device__ __forceinline__ void emit_shadow(const PathState& P, const DeviceScen
         P.sh_o[q] = make_float4(so.x, so.y, so.z, env ? -tmax : tmax);
         P.sh_d[q] = make_float4(d.x, d.y, d.z, __int_as_float(slot));
         P.sh_c[q] = make_float4(c.x, c.y, c.z, __int_as_float(rec));
+        if (P.sort.place[0]) ray_place(S, P.sort, 0, (uint32_t)q, so, d);
     } else {
         // c rounded before it is added, as k_shadow adds it from the queue: the
         // same image whichever kernel takes a bounce
@@ -433,6 +438,7 @@ __device__ __forceinline__ bool shade_one(const PathState& P, const DeviceScene&
     if (!TAIL) {
         int q = warp_append(true, &P.counters[CNT_OUT]);
         P.queue_out[q] = slot;
+        if (P.sort.place[1]) ray_place(S, P.sort, 1, (uint32_t)q, no, wi);
     }
     P.ray_o[slot] = make_float4(no.x, no.y, no.z, 0.f);
     P.ray_d[slot] = make_float4(wi.x, wi.y, wi.z, env_sampled ? pdf : 0.f);
@@ -551,7 +557,7 @@ __global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_M
             const f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
             float t, b1, b2;
             const int tri = WALK == 3   ? closest_hit_wide<false>(S, o, d, t, b1, b2)
-                            : WALK == 2 ? closest_hit_fast(S, o, d, t, b1, b2)
+                            : WALK == 2 ? closest_hit_fast<true>(S, o, d, t, b1, b2)
                                         : closest_hit_ww(S, o, d, t, b1, b2);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
             ++rays;
@@ -561,6 +567,16 @@ __global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_M
     }
     warp_count(rays, &P.counters[CNT_RAYS]);
     warp_count(shadows, &P.counters[CNT_SHRAYS]);
+}
+
+// The two queues of a sorted bounce: blockIdx.y 0 writes the order of the
+// shadow queue, 1 the continuing paths into queue_out.
+__global__ void k_ray_order(PathState P) {
+    const int which = blockIdx.y;
+    const uint32_t n = which ? P.counters[CNT_OUT] : min(P.counters[CNT_SHADOW], (uint32_t)P.sh_cap);
+    int32_t* __restrict__ to = which ? P.queue_out : P.sort.order;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+        to[ray_offset(P.sort, which, q)] = which ? P.sort.queue[q] : (int32_t)q;
 }
 
 // ---------------------------------------------------------------- shadow rays
@@ -752,7 +768,7 @@ static int g_trace_blocks = 0, g_shadow_blocks = 0, g_num_sms = 1;
 void launch_setup(int num_sms) {
     g_num_sms = num_sms > 0 ? num_sms : 1;
     int b1 = 0, b2 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_trace<false, true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_trace<false, 1>, 128, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k_shadow<false, true>, 128, 0);
     g_trace_blocks = num_sms * (b1 > 0 ? b1 : 1);
     g_shadow_blocks = num_sms * (b2 > 0 ? b2 : 1);
@@ -767,12 +783,15 @@ static int count_grid(int cap);
 
 void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, int max_count,
                    cudaStream_t st, cudaEvent_t* ev, bool count, const NrcCtx* nrc) {
+    const bool sorted = P.sort.place[0] != nullptr;
     if (ev) cudaEventRecord(ev[0], st);
-    switch ((count ? 2 : 0) + pol.trav) {
-        case 0: k_trace<false, false><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
-        case 1: k_trace<false, true><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
-        case 2: k_trace<true, false><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
-        default: k_trace<true, true><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+    switch ((count ? 3 : 0) + (pol.trav ? 1 + P.sort.input : 0)) {
+        case 0: k_trace<false, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 1: k_trace<false, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 2: k_trace<false, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 3: k_trace<true, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 4: k_trace<true, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        default: k_trace<true, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
     }
     if (ev) cudaEventRecord(ev[1], st);
     // the shading kernels stride over their device counts; max_count (an
@@ -781,8 +800,18 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
     if (shade_blocks < 1) shade_blocks = 1;
     const int most = g_num_sms * NR_SHADE_MINB * NR_SHADE_ROUNDS;
     if (shade_blocks > most) shade_blocks = most;
-    if (nrc) launch_shade<true>(P, S, pol, capacity, shade_blocks, *nrc, st);
-    else launch_shade<false>(P, S, pol, capacity, shade_blocks, NrcCtx{}, st);
+    PathState Q = P;
+    if (sorted) {  // shading appends the continuing paths beside, the sort moves them into queue_out
+        Q.queue_out = P.sort.queue;
+        for (int k = 0; k < 2; ++k) cudaMemsetAsync(P.sort.hist[k], 0, (size_t)P.sort.buckets() * 4, st);
+    }
+    if (nrc) launch_shade<true>(Q, S, pol, capacity, shade_blocks, *nrc, st);
+    else launch_shade<false>(Q, S, pol, capacity, shade_blocks, NrcCtx{}, st);
+    if (sorted) {
+        k_ray_scan<<<dim3(P.sort.buckets() / 4096u, 2), 1024, 0, st>>>(P.sort);
+        k_ray_scan_parts<<<2, 1024, 0, st>>>(P.sort);
+        k_ray_order<<<dim3(g_num_sms * 4, 2), 256, 0, st>>>(P);
+    }
     if (ev) cudaEventRecord(ev[2], st);
     float4* tb = (nrc && nrc->direct) ? nrc->t_before : nullptr;
     switch ((count ? 2 : 0) + pol.trav) {
@@ -816,8 +845,8 @@ void launch_tail(const PathState& P, const DeviceScene& S, const Policy& pol, in
 }
 
 void launch_trace(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, cudaStream_t st) {
-    if (pol.trav) k_trace<false, true><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
-    else k_trace<false, false><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
+    if (pol.trav) k_trace<false, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
+    else k_trace<false, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
 }
 void launch_advance(uint32_t* counters, cudaStream_t st) { k_advance<<<1, 1, 0, st>>>(counters); }
 int shadow_grid() { return g_shadow_blocks; }

@@ -70,7 +70,9 @@ void launch_raygen(const PathState& P, const WaveDesc& W, const nr_camera& cam, 
 // trace + sort, shade (for waves above 2^22 paths one kernel per shading
 // category the scene's materials can produce, else one for all), shadow,
 // (envis: the environment samples' fold), advance: bounce_launches(capacity,
-// envis, scene category mask) kernels. ev (optional) receives 4 events.
+// envis, scene category mask) kernels, and SORT_LAUNCHES more with P.sort (the
+// bounce's new rays sorted, ray_sort.cuh). ev (optional) receives 4 events.
+constexpr int SORT_LAUNCHES = 3;
 constexpr int SHADE_SPLIT_MIN = 1 << 22;
 inline int bounce_launches(int capacity, bool envis, uint32_t cat_mask) {
     return (capacity > SHADE_SPLIT_MIN ? 3 + __builtin_popcount(cat_mask) : 4) + (envis ? 1 : 0);

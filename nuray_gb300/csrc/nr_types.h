@@ -126,6 +126,21 @@ struct SlotField {
     __host__ __device__ T& operator[](size_t i) const { return p[2 * i]; }
 };
 
+// The sort of a bounce's new rays (ray_sort.cuh): [0] the shadow queue, [1]
+// the continuing paths. place null: rays stay in queue order.
+struct RaySort {
+    uint2* place[2];      // (bucket, place in it) of each entry
+    uint32_t* hist[2];    // bucket sizes, then offsets
+    uint32_t* part[2];    // per 4096 buckets
+    int32_t* order;       // the shadow queue's entries in sorted order
+    int32_t* queue;       // continuing paths as shading appends them; queue_out receives them sorted
+    int32_t origin_bits;  // per axis
+    int32_t dir_bits;     // per axis of the octahedral map
+    float cells_per_unit;
+    int32_t input;        // 1: queue_in was sorted by the bounce before
+    __host__ __device__ uint32_t buckets() const { return 1u << (3 * origin_bits + 2 * dir_bits); }
+};
+
 // Wavefront path state, structure of arrays, one slot per in-flight path.
 struct PathState {
     SlotField<float4> ray_o;  // (origin, unused)
@@ -144,6 +159,7 @@ struct PathState {
     float4* sh_c;    // (contribution if unoccluded, training record)
     int32_t sh_cap;  // entries of the shadow-ray queue (1 or 2 per slot)
     uint8_t* vis;    // null, or per slot: 1 if its light sample of this bounce was unoccluded
+    RaySort sort;
     // device counters (see Counter)
     uint32_t* counters;
 };
