@@ -229,8 +229,8 @@ class Scene:
         o = np.ascontiguousarray(o, np.float32).reshape(-1, 3)
         d = np.ascontiguousarray(d, np.float32).reshape(-1, 3)
         n = o.shape[0]
-        tri = np.zeros(n, np.int32)
-        t, b1, b2 = (np.zeros(n, np.float32) for _ in range(3))
+        tri = np.empty(n, np.int32)  # outputs the library fills are not cleared first
+        t, b1, b2 = (np.empty(n, np.float32) for _ in range(3))
         check(lib().nr_intersect(self._h, n, _ptr(o), _ptr(d), _ptr(tri), _ptr(t), _ptr(b1), _ptr(b2),
                                  NR_INTERSECT_EXHAUSTIVE if exhaustive else 0))
         return tri, t, b1, b2
@@ -241,8 +241,8 @@ class Scene:
     def render(self, params, camera=None, want_rgb8=False, cancel=None, progress=None):
         cfg = parse_params(params)
         w, h = int(cfg.get("imgw", 1)), int(cfg.get("imgh", 1))
-        hdr = np.zeros((h, w, 3), np.float32)
-        rgb8 = np.zeros((h, w, 3), np.uint8) if want_rgb8 else None
+        hdr = np.empty((h, w, 3), np.float32)
+        rgb8 = np.empty((h, w, 3), np.uint8) if want_rgb8 else None
         cam = ctypes.byref(camera) if camera is not None else None
         cb = None
         if progress is not None:
@@ -260,7 +260,7 @@ class Scene:
 
     def render_samples(self, params, pix_xy, spp, sample0=0, camera=None):
         pix = np.ascontiguousarray(pix_xy, np.int32).reshape(-1, 2)
-        out = np.zeros((pix.shape[0], spp, 3), np.float32)
+        out = np.empty((pix.shape[0], spp, 3), np.float32)
         cam = ctypes.byref(camera) if camera is not None else None
         check(lib().nr_render_samples(self._h, cam, params.encode(), pix.shape[0], _ptr(pix), sample0, spp, _ptr(out)))
         return out
@@ -275,7 +275,7 @@ class Scene:
         """d loss / d (albedo rgb, roughness, emission rgb) per material, shape (num_mats, 7)."""
         d = np.ascontiguousarray(dl_dimage, np.float32)
         n = self.info()["mats"]
-        g = np.zeros((n, 7), np.float32)
+        g = np.empty((n, 7), np.float32)
         img = np.zeros(d.shape, np.float32) if want_image else None
         cam = ctypes.byref(camera) if camera is not None else None
         check(lib().nr_adjoint(self._h, cam, params.encode(), _ptr(d), _ptr(g), _ptr(img)))

@@ -39,7 +39,7 @@ class Cache:
             pass
 
     def get_params(self):
-        p = np.zeros(NUM_PARAMS, np.float32)
+        p = np.empty(NUM_PARAMS, np.float32)
         check(self.L.nr_nrc_get_params(self._h, _ptr(p)))
         return p
 
@@ -67,14 +67,14 @@ class Cache:
 
     def infer(self, x):
         x = np.ascontiguousarray(x, np.float32).reshape(-1, INPUTS)
-        out = np.zeros((x.shape[0], 3), np.float32)
+        out = np.empty((x.shape[0], 3), np.float32)
         check(self.L.nr_nrc_infer(self._h, x.shape[0], _ptr(x), _ptr(out)))
         return out
 
     def gradient(self, x, y):
         x = np.ascontiguousarray(x, np.float32).reshape(-1, INPUTS)
         y = np.ascontiguousarray(y, np.float32).reshape(-1, 3)
-        g = np.zeros(NUM_PARAMS, np.float32)
+        g = np.empty(NUM_PARAMS, np.float32)
         loss = ctypes.c_float()
         check(self.L.nr_nrc_gradient(self._h, x.shape[0], _ptr(x), _ptr(y), _ptr(g), ctypes.byref(loss)))
         return g, loss.value
