@@ -128,15 +128,16 @@ struct nr_nrc {
     __nv_bfloat16 *x = nullptr, *acts = nullptr, *dz = nullptr;
     float *y = nullptr, *out = nullptr, *loss = nullptr;
     float* xf = nullptr;  // FP32 staging of caller inputs
+    bool host_access = false;    // kernels may read and write the caller's host arrays
     float* loss_host = nullptr;  // pinned
     bool tc = true;              // inference on tcgen05 (nrc_tc.cu); false: mma.sync (nrc.cu)
     uint32_t tc_first_wait = NR_TC_FIRST_WAIT_LIMIT;  // bound of the first MMA wait of a layer
     // the tensor-core kernels, unless disabled here or, after an unfinished
     // MMA group (error bit 32), for the whole process
     bool use_tc() const { return tc && nr::nrc_tc_enabled(); }
-    DevBuf errbuf;               // error word of the tensor-core kernels
-    DevBuf wt_img;               // packed transposed weights of the tensor-core backward pass
-    uint32_t* err_host = nullptr;  // pinned
+    DevBuf errbuf;               // error word of the tensor-core kernels, then the loss sum
+    DevBuf wt_img;               // transposed weights of the tensor-core backward pass (dev.wt_img)
+    uint32_t* err_host = nullptr;  // pinned: the error word and the loss sum
 
     ~nr_nrc() {
         cudaSetDevice(device);
@@ -638,7 +639,7 @@ void nrc_ensure_batch(nr_nrc* c, int m) {
     if (m <= c->batch_cap) return;
     size_t M = (size_t)m;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    size_t bytes = al(M * NRC_IN * 2) + al(M * 12) + al(M * 12) + al(4 * M * NRC_H * 2) + al(5 * M * NRC_H * 2) + 256 +
+    size_t bytes = al(M * NRC_IN * 2) + al(M * 12) + al(M * 12) + al(4 * M * NRC_H * 2) + al(5 * M * NRC_H * 2) +
                    al(M * NRC_IN * 4);
     c->batch.alloc(bytes);
     char* p = c->batch.as<char>();
@@ -648,39 +649,29 @@ void nrc_ensure_batch(nr_nrc* c, int m) {
     c->out = (float*)take(M * 12);
     c->acts = (__nv_bfloat16*)take(4 * M * NRC_H * 2);
     c->dz = (__nv_bfloat16*)take(5 * M * NRC_H * 2);
-    c->loss = (float*)take(4);
     c->xf = (float*)take(M * NRC_IN * 4);
     c->batch_cap = m;
 }
 
-// Forward and backward of the rows R (gradients added to c->dev.grad, loss
-// to c->loss): on the tensor cores (tcgen05: forward and data gradients;
-// weight gradients by mma.sync) with tc, else all by mma.sync. err: the
-// word that receives bit 8 if a tensor-core wait timed out.
+// Backward of the rows R after a forward on the tensor cores (gradients added
+// to c->dev.grad, loss to c->loss): data gradients by tcgen05, weight
+// gradients by mma.sync. err: the word that receives bit 8 if a tensor-core
+// wait timed out.
+void nrc_backward(nr_nrc* c, const __nv_bfloat16* x, const float* y, const nr::NrcRows& R, uint32_t* err, cudaStream_t st) {
+    nr::nrc_launch_backward_data_tc(c->out, y, c->acts, c->dz, R, c->loss, c->num_sms, c->dev.wt_img, err, st,
+                                    c->tc_first_wait);
+    nr::nrc_launch_backward_weight(c->dev, x, c->dz, c->acts, R, c->num_sms, st);
+}
+// Forward and backward on the tensor cores with tc, else all by mma.sync.
 void nrc_forward_backward(nr_nrc* c, const __nv_bfloat16* x, const float* y, const nr::NrcRows& R, uint32_t* err,
                           cudaStream_t st) {
     if (c->use_tc()) {
         nr::nrc_launch_forward_tc(c->dev.wb, c->dev.params, x, R, c->out, c->num_sms, err, st, c->acts,
                                   c->tc_first_wait);
-        nr::nrc_launch_backward_data_tc(c->dev.wb, c->out, y, c->acts, c->dz, R, c->loss, c->num_sms, c->wt_img.p, err,
-                                        st, c->tc_first_wait);
-        nr::nrc_launch_backward_weight(c->dev, x, c->dz, c->acts, R, c->num_sms, st);
+        nrc_backward(c, x, y, R, err, st);
     } else {
         nr::nrc_launch_forward(c->dev, x, R, c->out, c->acts, c->num_sms, st);
         nr::nrc_launch_backward(c->dev, x, c->out, y, c->acts, c->dz, R, c->loss, c->num_sms, st);
-    }
-}
-
-// Gradient (and, when `update`, one Adam step) on m rows already on the
-// device: x BF16 [m][80], y [m][3]. Returns the summed loss asynchronously in c->loss.
-void nrc_train_device(nr_nrc* c, const __nv_bfloat16* x, const float* y, int m, bool update, cudaStream_t st) {
-    nrc_ensure_batch(c, m);
-    NR_CUDA(cudaMemsetAsync(c->loss, 0, 4, st));
-    const nr::NrcRows R = nr::nrc_rows(m);
-    nrc_forward_backward(c, x, y, R, c->errbuf.as<uint32_t>(), st);
-    if (update) {
-        c->step++;
-        nr::nrc_launch_adam(c->dev, c->lr, c->b1, c->b2, c->eps, c->step, c->ema, R, st, c->errbuf.as<uint32_t>());
     }
 }
 
@@ -1641,6 +1632,7 @@ int nr_nrc_create(const char* params, nr_nrc** out) {
         auto n = std::make_unique<nr_nrc>();
         NR_CUDA(cudaGetDevice(&n->device));
         NR_CUDA(cudaDeviceGetAttribute(&n->num_sms, cudaDevAttrMultiProcessorCount, n->device));
+        n->host_access = reads_host(n->device);
         NR_CUDA(cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking));
         NR_CUDA(cudaMallocHost(&n->loss_host, 4));
         n->lr = c.get_float("lr", 1e-3f);
@@ -1663,9 +1655,11 @@ int nr_nrc_create(const char* params, nr_nrc** out) {
         nr::nrc_setup();
         nr::nrc_tc_setup();
         n->errbuf.alloc(256);
-        n->wt_img.alloc(nr::nrc_wt_image_bytes());
+        n->loss = n->errbuf.as<float>() + 1;
+        n->wt_img.alloc(NRC_WT_BYTES);
+        n->dev.wt_img = n->wt_img.as<unsigned char>();
         NR_CUDA(cudaMemsetAsync(n->errbuf.p, 0, 4, n->stream));
-        NR_CUDA(cudaMallocHost(&n->err_host, 4));
+        NR_CUDA(cudaMallocHost(&n->err_host, 8));
         const size_t P = NRC_NUM_PARAMS;
         n->pbuf.alloc(6 * P * 4 + 2 * P * 2 + 512);
         float* f = n->pbuf.as<float>();
@@ -1695,7 +1689,7 @@ int nr_nrc_create(const char* params, nr_nrc** out) {
         NR_CUDA(cudaMemcpyAsync(n->dev.params, init.data(), P * 4, cudaMemcpyHostToDevice, n->stream));
         NR_CUDA(cudaMemcpyAsync(n->dev.pinf, init.data(), P * 4, cudaMemcpyHostToDevice, n->stream));
         NR_CUDA(cudaMemsetAsync(n->dev.grad, 0, 4 * P * 4, n->stream));  // grad, m, v, ema
-        nr::nrc_launch_to_bf16(n->dev.params, n->dev.wb, P, n->stream);
+        nr::nrc_launch_refresh(n->dev, n->stream);
         nr::nrc_launch_to_bf16(n->dev.params, n->dev.wb_inf, P, n->stream);
         NR_CUDA(cudaStreamSynchronize(n->stream));
         *out = n.release();
@@ -1724,7 +1718,7 @@ int nr_nrc_set_params(nr_nrc* n, const float* in) {
         NR_CUDA(cudaMemcpyAsync(n->dev.params, in, NRC_NUM_PARAMS * 4, cudaMemcpyHostToDevice, n->stream));
         NR_CUDA(cudaMemcpyAsync(n->dev.pinf, in, NRC_NUM_PARAMS * 4, cudaMemcpyHostToDevice, n->stream));
         NR_CUDA(cudaMemsetAsync(n->dev.grad, 0, 4 * (size_t)NRC_NUM_PARAMS * 4, n->stream));
-        nr::nrc_launch_to_bf16(n->dev.params, n->dev.wb, NRC_NUM_PARAMS, n->stream);
+        nr::nrc_launch_refresh(n->dev, n->stream);
         nr::nrc_launch_to_bf16(n->dev.params, n->dev.wb_inf, NRC_NUM_PARAMS, n->stream);
         n->step = 0;
         NR_CUDA(cudaStreamSynchronize(n->stream));
@@ -1796,7 +1790,7 @@ int nr_nrc_set_state(nr_nrc* n, int32_t which, const float* in) {
         }
         NR_CUDA(cudaMemcpyAsync(dst, in, P * 4, cudaMemcpyHostToDevice, n->stream));
         // the BF16 copies the kernels read follow their FP32 sources
-        if (which == NR_NRC_STATE_PARAMS) nr::nrc_launch_to_bf16(n->dev.params, n->dev.wb, P, n->stream);
+        if (which == NR_NRC_STATE_PARAMS) nr::nrc_launch_refresh(n->dev, n->stream);
         if (which == NR_NRC_STATE_INFER) nr::nrc_launch_to_bf16(n->dev.pinf, n->dev.wb_inf, P, n->stream);
         NR_CUDA(cudaStreamSynchronize(n->stream));
         NR_CUDA(cudaGetLastError());
@@ -1819,11 +1813,14 @@ void nrc_check_err(nr_nrc* c, const char* what) {
                                      ": " + nr::err_bits_text() + ")");
 }
 
-// Uploads n rows of FP32 inputs and converts them to BF16 in the batch scratch.
-void nrc_upload_x(nr_nrc* c, int n, const float* x) {
+// n rows of FP32 inputs where a kernel can read them: the caller's array, or
+// its copy in the batch scratch where the device cannot read that in place
+// (or not in 16-byte pieces).
+const float* nrc_rows_f32(nr_nrc* c, int n, const float* x) {
     nrc_ensure_batch(c, n);
+    if (c->host_access && (reinterpret_cast<uintptr_t>(x) & 15) == 0) return x;
     NR_CUDA(cudaMemcpyAsync(c->xf, x, (size_t)n * NRC_IN * 4, cudaMemcpyHostToDevice, c->stream));
-    nr::nrc_launch_to_bf16(c->xf, c->x, (size_t)n * NRC_IN, c->stream);
+    return c->xf;
 }
 }  // namespace
 
@@ -1833,13 +1830,17 @@ int nr_nrc_infer(nr_nrc* c, int32_t n, const float* x, float* out) {
         if (n == 0) return;
         std::lock_guard<std::mutex> lk(c->mu);
         NR_CUDA(cudaSetDevice(c->device));
-        nrc_upload_x(c, n, x);
-        if (c->use_tc())
-            nr::nrc_launch_forward_tc(c->dev.wb, c->dev.params, c->x, nr::nrc_rows(n), c->out, c->num_sms,
-                                      c->errbuf.as<uint32_t>(), c->stream, nullptr, c->tc_first_wait);
-        else
-            nr::nrc_launch_forward(c->dev, c->x, nr::nrc_rows(n), c->out, nullptr, c->num_sms, c->stream);
-        NR_CUDA(cudaMemcpyAsync(out, c->out, (size_t)n * 12, cudaMemcpyDeviceToHost, c->stream));
+        const float* xf = nrc_rows_f32(c, n, x);
+        float* to = c->host_access ? out : c->out;
+        if (c->host_access) touch_pages(out, (size_t)n * 12);
+        if (c->use_tc()) {
+            nr::nrc_launch_forward_tc_f32(c->dev.wb, c->dev.params, xf, nullptr, nr::nrc_rows(n), to, c->num_sms,
+                                          c->errbuf.as<uint32_t>(), c->stream, nullptr, c->tc_first_wait, nullptr);
+        } else {
+            nr::nrc_launch_to_bf16(xf, c->x, (size_t)n * NRC_IN, c->stream);
+            nr::nrc_launch_forward(c->dev, c->x, nr::nrc_rows(n), to, nullptr, c->num_sms, c->stream);
+        }
+        if (!c->host_access) NR_CUDA(cudaMemcpyAsync(out, c->out, (size_t)n * 12, cudaMemcpyDeviceToHost, c->stream));
         NR_CUDA(cudaMemcpyAsync(c->err_host, c->errbuf.p, 4, cudaMemcpyDeviceToHost, c->stream));
         NR_CUDA(cudaStreamSynchronize(c->stream));
         NR_CUDA(cudaGetLastError());
@@ -1852,23 +1853,35 @@ static int nrc_grad_impl(nr_nrc* c, int32_t n, const float* x, const float* y, f
         if (!c || n <= 0 || !x || !y) throw NrError(NR_ERR_INVALID, "bad argument");
         std::lock_guard<std::mutex> lk(c->mu);
         NR_CUDA(cudaSetDevice(c->device));
-        nrc_upload_x(c, n, x);
-        NR_CUDA(cudaMemcpyAsync(c->y, y, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
-        nrc_train_device(c, c->x, c->y, n, false, c->stream);
+        const float* xf = nrc_rows_f32(c, n, x);
+        const float* yd = y;
+        if (!c->host_access) {
+            NR_CUDA(cudaMemcpyAsync(c->y, y, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
+            yd = c->y;
+        }
+        const nr::NrcRows R = nr::nrc_rows(n);
+        uint32_t* err = c->errbuf.as<uint32_t>();
+        if (c->use_tc()) {
+            nr::nrc_launch_forward_tc_f32(c->dev.wb, c->dev.params, xf, c->x, R, c->out, c->num_sms, err, c->stream, c->acts,
+                                          c->tc_first_wait, c->loss);
+            nrc_backward(c, c->x, yd, R, err, c->stream);
+        } else {
+            nr::nrc_launch_to_bf16(xf, c->x, (size_t)n * NRC_IN, c->stream);
+            NR_CUDA(cudaMemsetAsync(c->loss, 0, 4, c->stream));
+            nrc_forward_backward(c, c->x, yd, R, err, c->stream);
+        }
         if (grad) NR_CUDA(cudaMemcpyAsync(grad, c->dev.grad, NRC_NUM_PARAMS * 4, cudaMemcpyDeviceToHost, c->stream));
         if (update) {
             c->step++;
-            nr::nrc_launch_adam(c->dev, c->lr, c->b1, c->b2, c->eps, c->step, c->ema, nr::nrc_rows(n), c->stream,
-                                c->errbuf.as<uint32_t>());
+            nr::nrc_launch_adam(c->dev, c->lr, c->b1, c->b2, c->eps, c->step, c->ema, R, c->stream, err);
         } else {
             NR_CUDA(cudaMemsetAsync(c->dev.grad, 0, NRC_NUM_PARAMS * 4, c->stream));
         }
-        NR_CUDA(cudaMemcpyAsync(c->loss_host, c->loss, 4, cudaMemcpyDeviceToHost, c->stream));
-        NR_CUDA(cudaMemcpyAsync(c->err_host, c->errbuf.p, 4, cudaMemcpyDeviceToHost, c->stream));
+        NR_CUDA(cudaMemcpyAsync(c->err_host, c->errbuf.p, 8, cudaMemcpyDeviceToHost, c->stream));
         NR_CUDA(cudaStreamSynchronize(c->stream));
         NR_CUDA(cudaGetLastError());
         nrc_check_err(c, "training");
-        if (loss) *loss = *c->loss_host;
+        if (loss) std::memcpy(loss, &c->err_host[1], 4);
     });
 }
 

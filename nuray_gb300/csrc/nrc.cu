@@ -58,6 +58,11 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Adds two floats to an 8-byte aligned pair in one reduction.
+__device__ __forceinline__ void red_add2(float* p, float a, float b) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(a), "f"(b) : "memory");
+}
+
 // Copies the BF16 weights into shared memory with padded strides; rows
 // 8..15 of W4 are zero.
 __device__ void load_weights(const __nv_bfloat16* __restrict__ wb, __nv_bfloat16* sm) {
@@ -382,22 +387,17 @@ __global__ void __launch_bounds__(128) k_nrc_backward_weight(const __nv_bfloat16
     for (int jt = 0; jt < 10; ++jt) {
         if (jt >= KT) break;
         const int c = 8 * jt + 2 * t;
-        if (n0 + g < N) {
-            atomicAdd(&gW[(n0 + g) * K + c], acc[jt][0]);
-            atomicAdd(&gW[(n0 + g) * K + c + 1], acc[jt][1]);
-        }
-        if (n0 + g + 8 < N) {
-            atomicAdd(&gW[(n0 + g + 8) * K + c], acc[jt][2]);
-            atomicAdd(&gW[(n0 + g + 8) * K + c + 1], acc[jt][3]);
-        }
+        // (pairs of columns: every layer starts at an even offset, K and c are even)
+        if (n0 + g < N) red_add2(&gW[(n0 + g) * K + c], acc[jt][0], acc[jt][1]);
+        if (n0 + g + 8 < N) red_add2(&gW[(n0 + g + 8) * K + c], acc[jt][2], acc[jt][3]);
     }
 }
 
-// Adam on the FP32 master parameters (Kingma & Ba), refreshing the BF16 copy
-// and clearing the gradient.
+// Adam on the FP32 master parameters (Kingma & Ba), refreshing the BF16 copy,
+// its transposed image and clearing the gradient.
 // Also advances the moving average used for inference: ema = beta ema +
 // (1 - beta) p, read with the start-up correction 1 / (1 - beta^t).
-__global__ void k_nrc_adam(float* __restrict__ p, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
+__global__ void k_nrc_adam(unsigned char* __restrict__ wt_img, float* __restrict__ p, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
                            __nv_bfloat16* __restrict__ wb, float* __restrict__ ema, float* __restrict__ pinf,
                            __nv_bfloat16* __restrict__ wb_inf, int n, float lr, float b1, float b2, float eps, float c1,
                            float c2, float beta, float cema, NrcRows R, const uint32_t* err) {
@@ -415,6 +415,8 @@ __global__ void k_nrc_adam(float* __restrict__ p, float* __restrict__ grad, floa
     float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     p[i] = pi;
     wb[i] = __float2bfloat16(pi);
+    const int at = nrc_wt_offset(i);
+    if (at >= 0) *reinterpret_cast<__nv_bfloat16*>(wt_img + at) = __float2bfloat16(pi);
     grad[i] = 0.f;
     float e = beta * ema[i] + (1.f - beta) * pi;
     ema[i] = e;
@@ -426,6 +428,15 @@ __global__ void k_nrc_adam(float* __restrict__ p, float* __restrict__ grad, floa
 __global__ void k_f32_to_bf16(const float* __restrict__ a, __nv_bfloat16* __restrict__ b, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) b[i] = __float2bfloat16(a[i]);
+}
+
+__global__ void k_nrc_refresh(const float* __restrict__ p, __nv_bfloat16* __restrict__ wb, unsigned char* __restrict__ wt_img) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= NRC_NUM_PARAMS) return;
+    const __nv_bfloat16 v = __float2bfloat16(p[i]);
+    wb[i] = v;
+    const int at = nrc_wt_offset(i);
+    if (at >= 0) *reinterpret_cast<__nv_bfloat16*>(wt_img + at) = v;
 }
 
 // ------------------------------------------------------------------ launchers
@@ -453,6 +464,16 @@ void nrc_launch_forward(const NrcDev& N, const __nv_bfloat16* x, const NrcRows& 
     k_nrc_forward<<<grid_for((M + 15) / 16, num_sms), 128, nrc_forward_smem(), st>>>(N.wb, N.params, x, R, out, acts);
 }
 
+// Blocks per layer of the weight gradients: each adds its 64 x 80 sums to the
+// gradient once, so more of them pay in atomics what fewer pay in rounds (us a
+// training step of 16,384 / 65,536 rows: 304 blocks 114 / 252, 152 112 / 248,
+// 61 123 / 285, 16 159 / 469; with single-float atomics before 30 us for the
+// kernel of 16,384 rows).
+static int weight_blocks(int M, int num_sms) {
+    const int chunks = (M + 63) / 64;
+    return chunks < num_sms ? chunks : num_sms;
+}
+
 void nrc_launch_backward(const NrcDev& N, const __nv_bfloat16* x, const float* out, const float* y,
                          const __nv_bfloat16* acts, __nv_bfloat16* dz, const NrcRows& R, float* loss_sum, int num_sms,
                          cudaStream_t st) {
@@ -460,8 +481,7 @@ void nrc_launch_backward(const NrcDev& N, const __nv_bfloat16* x, const float* o
     if (M <= 0) return;
     k_nrc_backward_data<<<grid_for((M + 15) / 16, num_sms), 128, nrc_backward_smem(), st>>>(N.wb, out, y, acts, R, dz,
                                                                                           loss_sum);
-    int blocks = (M + 63) / 64;
-    if (blocks > num_sms * 2) blocks = num_sms * 2;
+    const int blocks = weight_blocks(M, num_sms);
     k_nrc_backward_weight<<<dim3(blocks, 5), 128, 0, st>>>(dz, x, acts, R, N.grad);
 }
 
@@ -469,8 +489,7 @@ void nrc_launch_backward_weight(const NrcDev& N, const __nv_bfloat16* x, const _
                                 const __nv_bfloat16* acts, const NrcRows& R, int num_sms, cudaStream_t st) {
     const int M = max_rows(R);
     if (M <= 0) return;
-    int blocks = (M + 63) / 64;
-    if (blocks > num_sms * 2) blocks = num_sms * 2;
+    const int blocks = weight_blocks(M, num_sms);
     k_nrc_backward_weight<<<dim3(blocks, 5), 128, 0, st>>>(dz, x, acts, R, N.grad);
 }
 
@@ -478,7 +497,7 @@ void nrc_launch_adam(const NrcDev& N, float lr, float b1, float b2, float eps, i
                      const NrcRows& R, cudaStream_t st, const uint32_t* err) {
     float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
     float cema = 1.f - powf(ema_beta, (float)step);
-    k_nrc_adam<<<(NRC_NUM_PARAMS + 255) / 256, 256, 0, st>>>(N.params, N.grad, N.m, N.v, N.wb, N.ema, N.pinf, N.wb_inf,
+    k_nrc_adam<<<(NRC_NUM_PARAMS + 255) / 256, 256, 0, st>>>(N.wt_img, N.params, N.grad, N.m, N.v, N.wb, N.ema, N.pinf, N.wb_inf,
                                                             NRC_NUM_PARAMS, lr, b1, b2, eps, c1, c2, ema_beta, cema, R,
                                                             err);
 }
@@ -488,6 +507,11 @@ void nrc_launch_forward_inf(const NrcDev& N, const __nv_bfloat16* x, const NrcRo
     const int M = max_rows(R);
     if (M <= 0) return;
     k_nrc_forward<<<grid_for((M + 15) / 16, num_sms), 128, nrc_forward_smem(), st>>>(N.wb_inf, N.pinf, x, R, out, nullptr);
+}
+
+void nrc_launch_refresh(const NrcDev& N, cudaStream_t st) {
+    cudaMemsetAsync(N.wt_img, 0, NRC_WT_BYTES, st);  // W4's padding
+    k_nrc_refresh<<<(NRC_NUM_PARAMS + 255) / 256, 256, 0, st>>>(N.params, N.wb, N.wt_img);
 }
 
 void nrc_launch_to_bf16(const float* a, __nv_bfloat16* b, size_t n, cudaStream_t st) {

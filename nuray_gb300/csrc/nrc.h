@@ -36,7 +36,32 @@ struct NrcDev {
     float* ema;
     float* pinf;
     __nv_bfloat16* wb_inf;
+    // the transposed weights of wb as k_nrc_backward_data_tc's shared memory
+    // holds them (nrc_wt_offset); every write of wb keeps it in step
+    unsigned char* wt_img;
 };
+
+// Byte offset in the transposed image of weight i of the parameter vector
+// (W1..W4), or -1 for the others. B[n][k] = W[k][n] in the K-major layout of
+// 8 x 16-byte blocks, W4's 8 rows padded to K = 16.
+#define NRC_WT_W4 0
+#define NRC_WT_W3 (NRC_WT_W4 + (NRC_H / 8) * 2 * 128)
+#define NRC_WT_W2 (NRC_WT_W3 + (NRC_H / 8) * (NRC_H / 8) * 128)
+#define NRC_WT_W1 (NRC_WT_W2 + (NRC_H / 8) * (NRC_H / 8) * 128)
+#define NRC_WT_BYTES (NRC_WT_W1 + (NRC_H / 8) * (NRC_H / 8) * 128)
+#ifdef __CUDACC__
+__device__ __forceinline__ int nrc_wt_offset(int i) {
+    int base, at, kc;
+    if (i >= NRC_OFF_W4) { base = NRC_WT_W4; at = i - NRC_OFF_W4; kc = 2; if (at >= NRC_OUT_PAD * NRC_H) return -1; }
+    else if (i >= NRC_OFF_W3) { base = NRC_WT_W3; at = i - NRC_OFF_W3; kc = NRC_H / 8; }
+    else if (i >= NRC_OFF_W2) { base = NRC_WT_W2; at = i - NRC_OFF_W2; kc = NRC_H / 8; }
+    else if (i >= NRC_OFF_W1) { base = NRC_WT_W1; at = i - NRC_OFF_W1; kc = NRC_H / 8; }
+    else return -1;
+    if (kc != 2 && at >= NRC_H * NRC_H) return -1;  // a bias
+    const int k = at / NRC_H, n = at % NRC_H;
+    return base + (n / 8) * (kc * 128) + (k / 8) * 128 + (n % 8) * 16 + (k % 8) * 2;
+}
+#endif
 
 // The rows one launch works on. With count == nullptr they are [0, n). With
 // a device counter they are chunk `step` of `steps` equal chunks of
@@ -74,6 +99,8 @@ void nrc_launch_adam(const NrcDev& N, float lr, float b1, float b2, float eps, i
 void nrc_launch_forward_inf(const NrcDev& N, const __nv_bfloat16* x, const NrcRows& R, float* out, int num_sms,
                             cudaStream_t st);
 void nrc_launch_to_bf16(const float* a, __nv_bfloat16* b, size_t n, cudaStream_t st);
+// wb and its transposed image from the FP32 parameters.
+void nrc_launch_refresh(const NrcDev& N, cudaStream_t st);
 
 // Polls of the tensor-core kernels' bounded mbarrier waits (about 40 ms of
 // polling on the GB300 before a wait counts as timed out).
@@ -91,6 +118,12 @@ void nrc_tc_setup();
 void nrc_launch_forward_tc(const __nv_bfloat16* wb, const float* params, const __nv_bfloat16* x, const NrcRows& R,
                            float* out, int num_sms, uint32_t* err, cudaStream_t st, __nv_bfloat16* acts = nullptr,
                            uint32_t first_wait = NR_TC_FIRST_WAIT_LIMIT);
+// The same over FP32 rows (16-byte aligned; in device memory, or in host
+// memory the device can read), kept in BF16 in x unless that is null; *zero
+// (may be null) = 0 for a loss sum of a later kernel.
+void nrc_launch_forward_tc_f32(const __nv_bfloat16* wb, const float* params, const float* xf, __nv_bfloat16* x,
+                               const NrcRows& R, float* out, int num_sms, uint32_t* err, cudaStream_t st,
+                               __nv_bfloat16* acts, uint32_t first_wait, float* zero);
 // The same over compact query records (nrc_encode.cuh, [rows][2]), expanded
 // in shared memory: 32 bytes read per row instead of 160.
 void nrc_launch_forward_tc_records(const __nv_bfloat16* wb, const float* params, const uint4* rec, const NrcRows& R,
@@ -106,12 +139,10 @@ bool nrc_tc_enabled();
 // Training on the tensor cores: the data gradients (dz [5][ld][64], loss)
 // of k_nrc_backward_data by tcgen05.mma; the weight gradients then come
 // from nrc_launch_backward_weight.
-// wt_img: nrc_wt_image_bytes() of device scratch for the packed transposed
-// weights.
-void nrc_launch_backward_data_tc(const __nv_bfloat16* wb, const float* out, const float* y, const __nv_bfloat16* acts,
-                                 __nv_bfloat16* dz, const NrcRows& R, float* loss_sum, int num_sms, void* wt_img,
+// wt_img: NrcDev::wt_img.
+void nrc_launch_backward_data_tc(const float* out, const float* y, const __nv_bfloat16* acts,
+                                 __nv_bfloat16* dz, const NrcRows& R, float* loss_sum, int num_sms, const unsigned char* wt_img,
                                  uint32_t* err, cudaStream_t st, uint32_t first_wait = NR_TC_FIRST_WAIT_LIMIT);
-size_t nrc_wt_image_bytes();
 // The weight-gradient half of nrc_launch_backward (k_nrc_backward_weight).
 void nrc_launch_backward_weight(const NrcDev& N, const __nv_bfloat16* x, const __nv_bfloat16* dz,
                                 const __nv_bfloat16* acts, const NrcRows& R, int num_sms, cudaStream_t st);

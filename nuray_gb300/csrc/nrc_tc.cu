@@ -159,14 +159,21 @@ __device__ __forceinline__ bool wg_sync_or(int id, bool v) {
 }  // namespace
 
 // rec (or null): compact records [rows][2] (nrc_encode.cuh) expanded into
-// the A tile in place of rows of x.
+// the A tile in place of rows of x. xf (or null): FP32 rows [rows][80],
+// 16-byte aligned, in place of x, which then receives them in BF16 (null:
+// not kept); they may lie in host memory that the device can read. A tile's
+// rows are read 16 bytes a thread in order, so that lines come over the link
+// once and the tiles in flight hide it: 65,536 rows from host memory 190 ->
+// 155 us a call against a copy, a conversion pass and the forward.
 template <int NWG>
 __global__ void __launch_bounds__(128 * NWG) k_nrc_forward_tc(const __nv_bfloat16* __restrict__ wb,
                                                               const float* __restrict__ params,
-                                                              const __nv_bfloat16* __restrict__ x,
-                                                              const uint4* __restrict__ rec, NrcRows R,
+                                                              __nv_bfloat16* __restrict__ x,
+                                                              const uint4* __restrict__ rec,
+                                                              const float* __restrict__ xf, NrcRows R,
                                                               float* __restrict__ out, __nv_bfloat16* __restrict__ acts,
-                                                              uint32_t* err, uint32_t first_wait) {
+                                                              uint32_t* err, uint32_t first_wait, float* zero) {
+    if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0.f;  // the loss sum of the pass that follows
     int m0, M;
     if (!R.count) {
         m0 = 0;
@@ -180,7 +187,8 @@ __global__ void __launch_bounds__(128 * NWG) k_nrc_forward_tc(const __nv_bfloat1
     const int tiles = (M + TM - 1) / TM;
     if ((int)blockIdx.x * NWG >= tiles) return;  // no warpgroup of this CTA has a tile: no tensor memory taken
     if (rec) rec += 2 * (size_t)m0;
-    else x += (size_t)m0 * IN;
+    if (xf) xf += (size_t)m0 * IN;
+    if (x) x += (size_t)m0 * IN;
     out += (size_t)m0 * 3;
     const size_t LS = (size_t)R.ld * H;  // one layer of acts
 
@@ -243,6 +251,23 @@ __global__ void __launch_bounds__(128 * NWG) k_nrc_forward_tc(const __nv_bfloat1
 #pragma unroll
                 for (int c = 0; c < KC_IN; ++c)
                     *reinterpret_cast<uint4*>(dst + c * 128) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+            } else if (xf) {
+                // 20 pieces of 4 floats a row, the tile's 2560 in order
+                constexpr int Q = IN / 4;
+                const float4* src = reinterpret_cast<const float4*>(xf) + (size_t)tile * TM * Q;
+                const int most = min(TM, M - tile * TM) * Q;
+                uint2* keep = x ? reinterpret_cast<uint2*>(x) + (size_t)tile * TM * Q : nullptr;
+#pragma unroll 5
+                for (int i = wtid; i < TM * Q; i += TM) {
+                    uint2 w = make_uint2(0u, 0u);
+                    if (i < most) {
+                        const float4 v = __ldg(src + i);
+                        w = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+                        if (keep) keep[i] = w;
+                    }
+                    const int rr = i / Q, c = i % Q;
+                    *reinterpret_cast<uint2*>(abuf + (rr / 8) * (KC_IN * 128) + (rr % 8) * 16 + (c / 2) * 128 + (c % 2) * 8) = w;
+                }
             } else {
 #pragma unroll
                 for (int c = 0; c < KC_IN; ++c) {
@@ -334,41 +359,17 @@ __global__ void __launch_bounds__(128 * NWG) k_nrc_forward_tc(const __nv_bfloat1
 // k_nrc_backward_data writes it (layer 4: 8 columns), for
 // k_nrc_backward_weight; loss_sum (may be null) += the mean loss.
 namespace {
-constexpr int BK_W4T = 0;                                  // 64 x 16
-constexpr int BK_W3T = BK_W4T + (H / 8) * 2 * 128;         // 64 x 64 each
-constexpr int BK_W2T = BK_W3T + (H / 8) * KC_H * 128;
-constexpr int BK_W1T = BK_W2T + (H / 8) * KC_H * 128;
-constexpr int BK_A = BK_W1T + (H / 8) * KC_H * 128;        // 128 x 64 (the first product uses 128 x 16)
+constexpr int BK_W4T = NRC_WT_W4;                          // 64 x 16
+constexpr int BK_W3T = NRC_WT_W3;                          // 64 x 64 each
+constexpr int BK_W2T = NRC_WT_W2;
+constexpr int BK_W1T = NRC_WT_W1;
+constexpr int BK_A = NRC_WT_BYTES;                         // 128 x 64 (the first product uses 128 x 16)
 constexpr int BK_BAR = BK_A + (TM / 8) * KC_H * 128;
 constexpr int BK_TOTAL = BK_BAR + 16;
 
-// W [k][n] (row-major, `n_in` columns, `k_real` rows, the rest zero) into
-// the canonical K-major layout of B[n][k] with K = kk, at dst + off.
-__device__ void load_wt(unsigned char* sm, int off, const __nv_bfloat16* __restrict__ w, int n_in, int k_real, int kk) {
-    const int kc = kk / 8;
-    // consecutive threads read consecutive elements of a row of W
-    for (int i = threadIdx.x; i < n_in * kk; i += blockDim.x) {
-        const int k = i / n_in, n = i % n_in;
-        const __nv_bfloat16 v = k < k_real ? w[(size_t)k * n_in + n] : __float2bfloat16(0.f);
-        *reinterpret_cast<__nv_bfloat16*>(sm + off + (n / 8) * (kc * 128) + (k / 8) * 128 + (n % 8) * 16 + (k % 8) * 2) = v;
-    }
-}
 }  // namespace
 
-// The four transposed weight images of k_nrc_backward_data_tc (one per
-// block), packed once per pass into `img` (BK_A bytes) from which every CTA
-// copies them.
-__global__ void k_nrc_pack_wt(const __nv_bfloat16* __restrict__ wb, unsigned char* __restrict__ img) {
-    switch (blockIdx.x) {
-        case 0: load_wt(img, BK_W4T, wb + NRC_OFF_W4, H, NRC_OUT_PAD, 16); break;
-        case 1: load_wt(img, BK_W3T, wb + NRC_OFF_W3, H, H, H); break;
-        case 2: load_wt(img, BK_W2T, wb + NRC_OFF_W2, H, H, H); break;
-        default: load_wt(img, BK_W1T, wb + NRC_OFF_W1, H, H, H); break;
-    }
-}
-
-__global__ void __launch_bounds__(128) k_nrc_backward_data_tc(const __nv_bfloat16* __restrict__ wb,
-                                                              const float* __restrict__ out,
+__global__ void __launch_bounds__(128) k_nrc_backward_data_tc(const float* __restrict__ out,
                                                               const float* __restrict__ y,
                                                               const __nv_bfloat16* __restrict__ acts, NrcRows R,
                                                               __nv_bfloat16* __restrict__ dz, float* loss_sum,
@@ -530,9 +531,9 @@ void nrc_tc_setup() {
 }
 
 namespace {
-void launch_forward_tc(const __nv_bfloat16* wb, const float* params, const __nv_bfloat16* x, const uint4* rec,
+void launch_forward_tc(const __nv_bfloat16* wb, const float* params, __nv_bfloat16* x, const uint4* rec, const float* xf,
                        const NrcRows& R, float* out, int num_sms, uint32_t* err, cudaStream_t st, __nv_bfloat16* acts,
-                       uint32_t first_wait) {
+                       uint32_t first_wait, float* zero) {
     const int M = R.count ? (R.n + R.steps - 1) / R.steps : R.n;
     if (M <= 0) return;
     const int tiles = (M + TM - 1) / TM;
@@ -540,8 +541,8 @@ void launch_forward_tc(const __nv_bfloat16* wb, const float* params, const __nv_
     // resident CTAs per SM by shared memory: 3 with one warpgroup (58 KB), 2 with two or three
     const int cap = num_sms * (kFwWg == 1 ? 3 : 2);
     if (blocks > cap) blocks = cap;
-    k_nrc_forward_tc<kFwWg><<<blocks, 128 * kFwWg, nrc_forward_tc_smem(), st>>>(wb, params, x, rec, R, out, acts, err,
-                                                                              first_wait);
+    k_nrc_forward_tc<kFwWg><<<blocks, 128 * kFwWg, nrc_forward_tc_smem(), st>>>(wb, params, x, rec, xf, R, out, acts,
+                                                                              err, first_wait, zero);
 }
 
 // Compact records -> BF16 rows of 80 (for the mma.sync forward).
@@ -560,12 +561,19 @@ __global__ void k_nrc_expand(const uint4* __restrict__ rec, NrcRows R, __nv_bflo
 void nrc_launch_forward_tc(const __nv_bfloat16* wb, const float* params, const __nv_bfloat16* x, const NrcRows& R,
                            float* out, int num_sms, uint32_t* err, cudaStream_t st, __nv_bfloat16* acts,
                            uint32_t first_wait) {
-    launch_forward_tc(wb, params, x, nullptr, R, out, num_sms, err, st, acts, first_wait);
+    launch_forward_tc(wb, params, const_cast<__nv_bfloat16*>(x), nullptr, nullptr, R, out, num_sms, err, st, acts, first_wait,
+                      nullptr);
 }
 
 void nrc_launch_forward_tc_records(const __nv_bfloat16* wb, const float* params, const uint4* rec, const NrcRows& R,
                                    float* out, int num_sms, uint32_t* err, cudaStream_t st, uint32_t first_wait) {
-    launch_forward_tc(wb, params, nullptr, rec, R, out, num_sms, err, st, nullptr, first_wait);
+    launch_forward_tc(wb, params, nullptr, rec, nullptr, R, out, num_sms, err, st, nullptr, first_wait, nullptr);
+}
+
+void nrc_launch_forward_tc_f32(const __nv_bfloat16* wb, const float* params, const float* xf, __nv_bfloat16* x,
+                               const NrcRows& R, float* out, int num_sms, uint32_t* err, cudaStream_t st,
+                               __nv_bfloat16* acts, uint32_t first_wait, float* zero) {
+    launch_forward_tc(wb, params, x, nullptr, xf, R, out, num_sms, err, st, acts, first_wait, zero);
 }
 
 void nrc_launch_expand(const uint4* rec, const NrcRows& R, __nv_bfloat16* x, int num_sms, cudaStream_t st) {
@@ -574,19 +582,16 @@ void nrc_launch_expand(const uint4* rec, const NrcRows& R, __nv_bfloat16* x, int
     k_nrc_expand<<<blocks, 256, 0, st>>>(rec, R, x);
 }
 
-size_t nrc_wt_image_bytes() { return (size_t)BK_A; }
-
-void nrc_launch_backward_data_tc(const __nv_bfloat16* wb, const float* out, const float* y, const __nv_bfloat16* acts,
-                                 __nv_bfloat16* dz, const NrcRows& R, float* loss_sum, int num_sms, void* wt_img,
+void nrc_launch_backward_data_tc(const float* out, const float* y, const __nv_bfloat16* acts,
+                                 __nv_bfloat16* dz, const NrcRows& R, float* loss_sum, int num_sms, const unsigned char* wt_img,
                                  uint32_t* err, cudaStream_t st, uint32_t first_wait) {
     const int M = R.count ? (R.n + R.steps - 1) / R.steps : R.n;
     if (M <= 0) return;
-    k_nrc_pack_wt<<<4, 256, 0, st>>>(wb, static_cast<unsigned char*>(wt_img));
     int blocks = (M + TM - 1) / TM;
     const int cap = num_sms * 4;  // 43 KB of shared memory and 64 tensor-memory columns per CTA
     if (blocks > cap) blocks = cap;
-    k_nrc_backward_data_tc<<<blocks, 128, BK_TOTAL, st>>>(wb, out, y, acts, R, dz, loss_sum,
-                                                          static_cast<const unsigned char*>(wt_img), err, first_wait);
+    k_nrc_backward_data_tc<<<blocks, 128, BK_TOTAL, st>>>(out, y, acts, R, dz, loss_sum,
+                                                          wt_img, err, first_wait);
 }
 
 }  // namespace nr
