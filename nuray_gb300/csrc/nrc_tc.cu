@@ -511,13 +511,12 @@ __global__ void __launch_bounds__(128) k_nrc_backward_data_tc(const float* __res
     }
 }
 
-// Warpgroups per CTA of the forward kernel (NR_NRC_FW_WG: 1, 2 or 3).
-#ifndef NR_NRC_FW_WG
-#define NR_NRC_FW_WG 3
-#endif
-constexpr int kFwWg = NR_NRC_FW_WG;
-static_assert(kFwWg >= 1 && kFwWg <= 3, "1 to 3 warpgroups per forward CTA");
-size_t nrc_forward_tc_smem() { return (size_t)fw_smem(kFwWg); }
+// Warpgroups per CTA of the forward kernel: three for predictions, whose rows
+// come in tens of thousands; one for training, whose tiles are few and then
+// take an SM each (us a training step of 1024 / 16,384 / 65,536 rows: 84 / 109 /
+// 242 with three, 73 / 97 / 237 with one; predictions for 65,536 rows 135 with
+// three, 142 with one).
+constexpr int kInferWg = 3, kTrainWg = 1;
 
 namespace {
 std::atomic<bool> g_tc_disabled{false};
@@ -526,7 +525,8 @@ void nrc_tc_disable() { g_tc_disabled.store(true); }
 bool nrc_tc_enabled() { return !g_tc_disabled.load(); }
 
 void nrc_tc_setup() {
-    cudaFuncSetAttribute(k_nrc_forward_tc<kFwWg>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nrc_forward_tc_smem());
+    cudaFuncSetAttribute(k_nrc_forward_tc<kInferWg>, cudaFuncAttributeMaxDynamicSharedMemorySize, fw_smem(kInferWg));
+    cudaFuncSetAttribute(k_nrc_forward_tc<kTrainWg>, cudaFuncAttributeMaxDynamicSharedMemorySize, fw_smem(kTrainWg));
     cudaFuncSetAttribute(k_nrc_backward_data_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, BK_TOTAL);
 }
 
@@ -537,12 +537,16 @@ void launch_forward_tc(const __nv_bfloat16* wb, const float* params, __nv_bfloat
     const int M = R.count ? (R.n + R.steps - 1) / R.steps : R.n;
     if (M <= 0) return;
     const int tiles = (M + TM - 1) / TM;
-    int blocks = (tiles + kFwWg - 1) / kFwWg;
-    // resident CTAs per SM by shared memory: 3 with one warpgroup (58 KB), 2 with two or three
-    const int cap = num_sms * (kFwWg == 1 ? 3 : 2);
-    if (blocks > cap) blocks = cap;
-    k_nrc_forward_tc<kFwWg><<<blocks, 128 * kFwWg, nrc_forward_tc_smem(), st>>>(wb, params, x, rec, xf, R, out, acts,
-                                                                              err, first_wait, zero);
+    if (acts) {
+        // resident CTAs per SM by shared memory: 3 with one warpgroup (58 KB), 2 with three
+        const int blocks = std::min((tiles + kTrainWg - 1) / kTrainWg, num_sms * 3);
+        k_nrc_forward_tc<kTrainWg><<<blocks, 128 * kTrainWg, fw_smem(kTrainWg), st>>>(wb, params, x, rec, xf, R, out, acts, err,
+                                                                                    first_wait, zero);
+    } else {
+        const int blocks = std::min((tiles + kInferWg - 1) / kInferWg, num_sms * 2);
+        k_nrc_forward_tc<kInferWg><<<blocks, 128 * kInferWg, fw_smem(kInferWg), st>>>(wb, params, x, rec, xf, R, out, acts, err,
+                                                                                    first_wait, zero);
+    }
 }
 
 // Compact records -> BF16 rows of 80 (for the mma.sync forward).
