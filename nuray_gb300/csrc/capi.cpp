@@ -605,11 +605,11 @@ void ensure_paths(nr_scene* s, int cap, int sh_mult = 1) {
 // 5.53 / 5.49. Bits an axis of the origin and of the direction: 132.7M paths
 // 4+3 130.0, 5+3 124.7, 6+2 124.5, 6+3 120.9; 8.3M 4+3 9.90, 5+3 9.67, 6+3 9.81.
 // Without room for the workspace the rays stay in queue order.
-void ensure_sort(nr_scene* s, int cap, int live, int sh_mult, nr::PathState& P) {
+void ensure_sort(nr_scene* s, int cap, int live, int sh_mult, bool wanted, nr::PathState& P) {
     nr::RaySort& R = P.sort;
     R.input = R.place[0] ? 1 : 0;  // what the bounce before did
     R.place[0] = R.place[1] = nullptr;
-    if (live < 4000000 || s->dev.num_tris < 16384) return;
+    if (!wanted || live < 4000000 || s->dev.num_tris < 16384) return;
     R.origin_bits = cap >= (1 << 24) && s->dev.num_tris >= (1 << 19) ? 6 : 5;
     R.dir_bits = 3;
     float ext = 0.f;
@@ -943,6 +943,18 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
         }
         nrc_ensure_batch(s->nrc, std::max(s->nrc_tcap, cap));
     }
+    // Where the order of a cache's training records decides what it learns from
+    // them (several Adam steps on consecutive chunks; more records than the
+    // table holds: all of renderer=nrc's), the vertices are shaded bounce by
+    // bounce in the order of the paths.
+    bool in_order = false;
+    if (use_nrc) {
+        const int depth_cap = A.pol.maxdepth > 0 ? A.pol.maxdepth : 16;
+        const double per_path = A.nrc_query && A.nrc_train_depth > 0 ? std::min(A.nrc_train_depth, depth_cap) : depth_cap;
+        const double paths = (double)cap / (double)s->nrc_ctx.train_stride;
+        in_order = A.pol.excl || A.nrc_steps > 1 || A.pol.maxdepth == 0 ||
+                   (paths + 6.0 * std::sqrt(paths) + 6.0) * per_path > (double)s->nrc_ctx.tcap;
+    }
     const float film_h = nr::film_height(A.cam);
     const nr::DeviceScene D = scene_for(s, A.prune);
     auto t0 = std::chrono::steady_clock::now();
@@ -990,7 +1002,8 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
         const bool stepwise = A.profile || A.count;  // these time or count the wavefront's own kernels
         // (Waves of more than 2^25 paths and bounded depth: their last bounces
         // are under 1 % of them, 140.3 against 140.4 ms, and stay as they are.)
-        const int tail_at = A.tail > 0 ? (cap <= nr::SHADE_SPLIT_MIN ? A.tail : kMaxBounces)
+        const int fixed_tail = in_order && A.tail < 0 ? 2 : A.tail;
+        const int tail_at = fixed_tail > 0 ? (cap <= nr::SHADE_SPLIT_MIN ? fixed_tail : kMaxBounces)
                             : (A.tail < 0 && (cap <= (1 << 25) || A.pol.maxdepth == 0) ? -1 : kMaxBounces);
         int live = W.count;     // an upper bound of the paths entering the bounce
         int reads = 0, taken = 0;  // live counts asked for and received
@@ -1014,7 +1027,7 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
                 ev_kind.push_back(-1); ev_kind.push_back(0); ev_kind.push_back(1); ev_kind.push_back(2);
                 nev += 4;
             }
-            ensure_sort(s, cap, live, s->sh_mult, P);
+            ensure_sort(s, cap, live, s->sh_mult, !in_order, P);
             nr::launch_bounce(P, D, A.pol, cap, live, st, A.profile ? evs : nullptr, A.count,
                               use_nrc ? &s->nrc_ctx : nullptr);
             std::swap(P.queue_in, P.queue_out);
@@ -1025,7 +1038,8 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
             // The count entering the next bounce, read back; the one asked for
             // a bounce earlier is taken now, while this bounce runs.
             const bool last = A.pol.maxdepth > 0 && bounce + 1 >= A.pol.maxdepth;
-            if (!last && (A.pol.maxdepth == 0 || (tail_at < 0 && !stepwise) || (live_sync > 0 && bounce + 1 >= live_sync))) {
+            if (!last && (A.pol.maxdepth == 0 || (tail_at < 0 && !stepwise) || P.sort.place[0] ||
+                          (live_sync > 0 && bounce + 1 >= live_sync))) {
                 NR_CUDA(cudaMemcpyAsync(&s->counters_host[nr::NUM_COUNTERS + (reads & 1)], s->ps.counters + nr::CNT_IN, 4,
                                         cudaMemcpyDeviceToHost, st));
                 NR_CUDA(cudaEventRecord(s->live_ev[reads & 1], st));
@@ -1182,7 +1196,7 @@ uint64_t adjoint_waves(nr_scene* s, const RenderArgs& A, int npix, const float* 
             const bool rec = bounce < depth_rec;
             P.hit = rec ? rec_hit + (size_t)bounce * C : s->ps.hit;
             P.vis = rec ? rec_vis + (size_t)bounce * C : nullptr;
-            ensure_sort(s, cap, live, s->sh_mult, P);
+            ensure_sort(s, cap, live, s->sh_mult, true, P);
             nr::launch_bounce(P, D, pol1, cap, live, st, nullptr, false, nullptr);
             std::swap(P.queue_in, P.queue_out);
             launches += nr::bounce_launches(cap, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
