@@ -876,16 +876,18 @@ constexpr int kMaxBounces = 4096;
 // shade whatever material each lane met, so the line lies lower where several
 // surface types occur, and lower still for a whole wave, whose bounces mostly
 // lie ahead. ms of the whole wave in the tail / two wavefront bounces first, 1M
-// triangles of one type: 261k paths 0.84 / 0.99, 518k 1.35 / 1.41, 1.04M 2.35 /
-// 2.10; sky and dielectrics: 61k 0.76 / 0.95, 123k 1.10 / 1.15, 184k 1.68 /
-// 1.34; every type: 61k 0.30 / 0.37, 184k 0.51 / 0.49; a room of four types:
-// 61k 0.30 / 0.34, 123k 0.51 / 0.45, 261k 1.01 / 0.81. Later bounces, the room,
-// 1.04M unbounded paths: 1.81 / 1.75 / 1.92 / 2.52 with the line at 50k / 150k /
-// 300k / 600k; every type, 522k: 0.86 / 0.84 / 0.77 / 0.97.
+// triangles of one type: 130k paths 0.50 / 0.82, 518k 1.16 / 1.38, 1.04M 2.05 /
+// 2.00; sky and dielectrics: 123k 1.09 / 1.17, 184k 1.27 / 1.06; every type: 61k
+// 0.39 / 0.43, 184k 0.42 / 0.37; a room of four types: 123k 0.44 / 0.47, 184k
+// 0.78 / 0.77. With the line for later bounces at 300k / 600k / 1M / 1.3M: one
+// type, 1.2M 2.46 / 2.34 / 2.32 / 2.45, 2.1M 3.42 / 3.43 / 3.29 / 3.28, 8.3M
+// 9.83 / 9.81 / 9.68 / 9.70; room, 1.0M unbounded, 1.72 / 1.82 / 1.87 / 2.20, and
+// 1.71 at 100k; every type, 522k: 0.72 at 300k, 0.81 at 100k.
 int64_t tail_limit(uint32_t cat_mask, int bounce) {
     const int surfaces = __builtin_popcount(cat_mask & ((1u << NR_MAT_LIGHT) - 1u));
-    if (surfaces <= 1) return 600000;
-    return bounce == 0 ? 100000 : (bounce == 1 ? 0 : 300000);
+    if (bounce == 1) return 0;
+    if (surfaces <= 1) return bounce == 0 ? 600000 : 1000000;
+    return bounce == 0 ? 130000 : 300000;
 }
 
 void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pix, int sample0, float4* film,

@@ -531,39 +531,63 @@ static void launch_shade(const PathState& P, const DeviceScene& S, const Policy&
 // us at 8 blocks, 178 at 6; 57,600 365 / 354; 522,240 of every material (about
 // half of them live at the tail) 730 / 716.
 #define NR_TAIL_MINB_WIDE 6
-// Paths of a warp: a warp walks for as long as its slowest ray in every
-// phase, so a few paths are spread over 16 warps per SM, and up to 8 warps
-// per SM before warps fill (the whole path in this kernel, 1M triangles, 3072
-// paths: 350 us with full warps, 263 / 238 / 227 / 214 over 4 / 8 / 16 / 32
-// warps per SM; 15,360 paths 354 / 314 / 289 / 315; the room of 36 triangles,
-// bound by issue slots at 61,440 paths: 510 / 509 / 570 / 633).
+// Paths a warp starts with: a warp walks for as long as its slowest ray in
+// every phase, so a few paths are spread over 16 warps per SM, and up to 8 warps
+// per SM before warps fill (a path per thread, 1M triangles, 3072 paths: 350 us
+// with full warps, 263 / 238 / 227 / 214 over 4 / 8 / 16 / 32 warps per SM;
+// 15,360 paths 354 / 314 / 289 / 315; the room of 36 triangles, bound by issue
+// slots at 61,440 paths: 510 / 509 / 570 / 633).
 #define NR_TAIL_WARPS 16
 __host__ __device__ inline uint32_t tail_paths_per_warp(uint32_t n, uint32_t sms) {
     const uint32_t wide = sms * NR_TAIL_WARPS, warps = n <= 8u * wide ? wide : wide / 2u;
     const uint32_t take = (n + warps - 1u) / warps;
     return take < 1u ? 1u : (take > 32u ? 32u : take);
 }
-// WALK: 1 exact, 2 fast, 3 four-wide.
+// WALK: 1 exact, 2 fast, 3 four-wide. A lane whose path has ended takes the
+// next one of the queue at once (a warp's 32 paths are not done before the
+// longest of them, and most end early: 518,400 paths 1346 us with a path per
+// thread, 1175 with refilled lanes; refilled once 8 / 16 / 32 lanes are idle
+// 1180 / 1197 / 1296).
 template <bool NRC, int WALK>
-__global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_MINB) k_tail(PathState P, DeviceScene S, Policy pol, NrcCtx C,
-                                                              uint32_t sms) {
+__global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_MINB) k_tail(PathState P, DeviceScene S, Policy pol,
+                                                                                              NrcCtx C, uint32_t sms) {
     const uint32_t n = P.counters[CNT_IN], take = tail_paths_per_warp(n, sms);
-    const uint32_t lane = threadIdx.x & 31u, i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5), lane = threadIdx.x & 31u;
+    const uint32_t first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
+    const uint32_t given = warps * take;  // paths the warps start with; the rest are taken as lanes fall idle
+    bool more = given < n;                // (uniform) whether there may be any left
+    int slot = lane < take && first < n ? P.queue_in[first] : -1;
+    int b = 0;
     uint32_t rays = 0, shadows = 0;
-    if (lane < take && i < n) {
-        const int slot = P.queue_in[i];
-        bool on = true;
-        for (int b = 0; on && b < NR_TAIL_MAX_BOUNCES; ++b) {
+    while (true) {
+        const unsigned idle = __ballot_sync(0xffffffffu, slot < 0);
+        if (more && idle) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&P.counters[CNT_WORK], (uint32_t)__popc(idle));
+            base = given + __shfl_sync(0xffffffffu, base, 0);
+            more = base + (uint32_t)__popc(idle) < n;
+            if (slot < 0) {
+                const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+                if (i < n) { slot = P.queue_in[i]; b = 0; }
+            }
+        }
+        if (!__any_sync(0xffffffffu, slot >= 0)) break;
+        if (slot >= 0) {
             const f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
             float t, b1, b2;
             const int tri = WALK == 3   ? closest_hit_wide<false>(S, o, d, t, b1, b2)
-                            : WALK == 2 ? closest_hit_fast<true>(S, o, d, t, b1, b2)
+                            : WALK == 2 ? closest_hit_fast<false>(S, o, d, t, b1, b2)
                                         : closest_hit_ww(S, o, d, t, b1, b2);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
             ++rays;
-            on = shade_one<NRC, -1, WALK>(P, S, pol, slot, C, &shadows);
+            bool on = shade_one<NRC, -1, WALK>(P, S, pol, slot, C, &shadows);
+            if (on && ++b >= NR_TAIL_MAX_BOUNCES) {  // bounce cap: the path did not end
+                atomicOr(&P.counters[CNT_ERR], (uint32_t)NR_ERRBIT_BOUNCES);
+                on = false;
+            }
+            if (!on) slot = -1;
         }
-        if (on) atomicOr(&P.counters[CNT_ERR], (uint32_t)NR_ERRBIT_BOUNCES);  // bounce cap: the path did not end
+        __syncwarp();
     }
     warp_count(rays, &P.counters[CNT_RAYS]);
     warp_count(shadows, &P.counters[CNT_SHRAYS]);
@@ -827,12 +851,11 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
 
 void launch_tail(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, const NrcCtx* nrc,
                  cudaStream_t st) {
-    // n <= capacity paths, so many to a warp: at most capacity / 32 warps or the
-    // warps they spread over, and never more than paths
-    const uint32_t sms = (uint32_t)g_num_sms;
-    const int blocks = std::max((capacity + 127) / 128, std::min(g_num_sms * NR_TAIL_WARPS / 4, (capacity + 3) / 4));
     // the four-wide walk up to the count where it stops paying
     const int walk = pol.trav == 0 ? 1 : (S.wide && capacity <= 300000 ? 3 : 2);
+    const uint32_t sms = (uint32_t)g_num_sms;
+    // one round of resident blocks, fewer where there is not a path for each warp
+    const int blocks = std::min(g_num_sms * (walk == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_MINB), (capacity + 3) / 4);
     const NrcCtx C = nrc ? *nrc : NrcCtx{};
     switch (walk + (nrc ? 3 : 0)) {
         case 1: k_tail<false, 1><<<blocks, 128, 0, st>>>(P, S, pol, C, sms); break;
