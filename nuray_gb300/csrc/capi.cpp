@@ -1035,12 +1035,12 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
             std::swap(P.queue_in, P.queue_out);
             S.bounces++;
             S.trace_launches++;
-            S.kernel_launches += nr::bounce_launches(cap, A.pol.envis != 0, s->dev.cat_mask) +
+            S.kernel_launches += nr::bounce_launches(use_nrc ? cap : live, A.pol.envis != 0, s->dev.cat_mask) +
                                  (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
             // The count entering the next bounce, read back; the one asked for
             // a bounce earlier is taken now, while this bounce runs.
             const bool last = A.pol.maxdepth > 0 && bounce + 1 >= A.pol.maxdepth;
-            if (!last && (A.pol.maxdepth == 0 || (tail_at < 0 && !stepwise) || P.sort.place[0] ||
+            if (!last && (A.pol.maxdepth == 0 || (tail_at < 0 && !stepwise) || cap > nr::SHADE_SPLIT_MIN ||
                           (live_sync > 0 && bounce + 1 >= live_sync))) {
                 NR_CUDA(cudaMemcpyAsync(&s->counters_host[nr::NUM_COUNTERS + (reads & 1)], s->ps.counters + nr::CNT_IN, 4,
                                         cudaMemcpyDeviceToHost, st));
@@ -1201,7 +1201,7 @@ uint64_t adjoint_waves(nr_scene* s, const RenderArgs& A, int npix, const float* 
             ensure_sort(s, cap, live, s->sh_mult, true, P);
             nr::launch_bounce(P, D, pol1, cap, live, st, nullptr, false, nullptr);
             std::swap(P.queue_in, P.queue_out);
-            launches += nr::bounce_launches(cap, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
+            launches += nr::bounce_launches(live, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
             if (!live_after(bounce, live)) break;
         }
         nr::launch_collect(s->ps, W, s->adj_L.as<float>(), A.spp, A.pol.imgw, st);

@@ -488,14 +488,16 @@ __global__ void __launch_bounds__(128, NR_SHADE_MINB) k_shade(PathState P, Devic
         shade_one<NRC>(P, S, pol, P.sorted[(size_t)c * capacity + (i - start[c])], C);
     }
 }
-// Waves of at most SHADE_SPLIT_MIN paths shade with the one kernel for all
-// categories: their bounces are short, and six mostly empty launches per
-// bounce cost more than the split saves (time to relMSE 1e-3 with 960x540
-// frames of 1 spp: 10.40 s with one kernel, 11.34 s with seven).
+// Bounces of at most SHADE_SPLIT_MIN paths shade with the one kernel for all
+// categories: they are short, and six mostly empty launches per bounce cost
+// more than the split saves (time to relMSE 1e-3 with 960x540 frames of 1 spp:
+// 10.40 s with one kernel, 11.34 s with seven; later bounces of a large wave,
+// the room at 640x480 x 16 spp: 5.06 ms with one, 5.22 with five). With the
+// cache the wave's size decides, so that its training records keep one order.
 template <bool NRC>
-static void launch_shade(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, int blocks,
+static void launch_shade(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, int paths, int blocks,
                          const NrcCtx& C, cudaStream_t st) {
-    if (capacity <= SHADE_SPLIT_MIN) {
+    if (paths <= SHADE_SPLIT_MIN) {
         k_shade<NRC, -1><<<blocks, 128, 0, st>>>(P, S, pol, capacity, C);
         return;
     }
@@ -829,8 +831,8 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
         Q.queue_out = P.sort.queue;
         for (int k = 0; k < 2; ++k) cudaMemsetAsync(P.sort.hist[k], 0, (size_t)P.sort.buckets() * 4, st);
     }
-    if (nrc) launch_shade<true>(Q, S, pol, capacity, shade_blocks, *nrc, st);
-    else launch_shade<false>(Q, S, pol, capacity, shade_blocks, NrcCtx{}, st);
+    if (nrc) launch_shade<true>(Q, S, pol, capacity, capacity, shade_blocks, *nrc, st);
+    else launch_shade<false>(Q, S, pol, capacity, max_count, shade_blocks, NrcCtx{}, st);
     if (sorted) {
         k_ray_scan<<<dim3(P.sort.buckets() / 4096u, 2), 1024, 0, st>>>(P.sort);
         k_ray_scan_parts<<<2, 1024, 0, st>>>(P.sort);
