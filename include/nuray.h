@@ -287,9 +287,11 @@ int nr_intersect_noalloc(nr_scene* scene, int32_t n, const float* o, const float
  * sample, default 0: renders of disjoint sample ranges are independent and
  * their films sum), tile (the order of a wave's paths; the image is the same
  * for every choice. 2, the default: each warp's 32 paths are tile_samples
- * consecutive samples of a tile of 32 / tile_samples pixels, tile_samples
- * by default the largest power of two up to 32 dividing spp, when the tile
- * divides the image; else 1: 8x4 pixel tiles of one sample when imgw % 8 ==
+ * consecutive samples of a tile of 32 / tile_samples pixels, tile_samples the
+ * largest power of two up to 32 dividing spp, when the tile divides the image
+ * and tile_samples is at least 8 or all of spp; else all samples of each pixel
+ * in turn, pixels in 8x4 tiles. With tile_samples given, that tile or, where it
+ * does not divide, as 1: 8x4 pixel tiles of one sample when imgw % 8 ==
  * 0 and imgh % 4 == 0; else or with 0: scanline order), live_sync (with
  * maxdepth: the bounce after which the live path count is read back each
  * bounce; -1, the default, 5 for waves of more than 2^22 paths and never

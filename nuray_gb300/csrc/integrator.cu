@@ -659,6 +659,23 @@ __global__ void k_film(PathState P, WaveDesc W, float4* film, int imgw) {
         if (any) film[pix] = acc;
         return;
     }
+    if (W.tiled == 3) {
+        ragged_pixel(p, (uint32_t)imgw, (uint32_t)(W.npix / imgw), x, y);
+        const uint64_t first = (uint64_t)p * (uint64_t)W.spp, past = first + (uint64_t)W.spp;
+        uint64_t g = first < W.base ? W.base : first;
+        const uint64_t stop = past < end ? past : end;
+        if (g >= stop) return;
+        const uint32_t pix = (uint32_t)y * (uint32_t)imgw + (uint32_t)x;
+        float4 acc = film[pix];
+        for (; g < stop; ++g) {
+            const float4 r = P.rad[g - W.base];
+            acc.x += smax(0.f, r.x);
+            acc.y += smax(0.f, r.y);
+            acc.z += smax(0.f, r.z);
+        }
+        film[pix] = acc;
+        return;
+    }
     frame_pixel(p, imgw, W.tiled, x, y);
     const uint32_t pix = (uint32_t)y * (uint32_t)imgw + (uint32_t)x;
     uint64_t s_first = W.base / (uint64_t)W.npix;

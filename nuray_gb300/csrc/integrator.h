@@ -13,8 +13,10 @@ struct WaveDesc {
     uint32_t sample0;
     const int32_t* pix_xy;  // device (x, y) list, or null for the full frame
     int32_t tiled;          // 0 scanline; 1 full frame in 8x4 pixel tiles (frame_pixel); 2 a warp of paths
-                            // holds g_s consecutive samples of a g_w x g_h pixel tile (g_s g_w g_h = 32)
+                            // holds g_s consecutive samples of a g_w x g_h pixel tile (g_s g_w g_h = 32);
+                            // 3 all samples of a pixel, pixels in 8x4 tiles of any frame (ragged_pixel)
     int32_t g_s, g_w, g_h;
+    int32_t spp;            // of the frame, for 3
 };
 
 #ifdef __CUDACC__
@@ -29,6 +31,17 @@ __device__ __forceinline__ void frame_pixel(uint32_t p, int w, int tiled, int& x
         x = (int)(p % (uint32_t)w);
         y = (int)(p / (uint32_t)w);
     }
+}
+
+// Pixel p of a w x h frame in 8x4 tiles, row-major, the last column and row of
+// them narrower and lower where the frame does not divide.
+__device__ __forceinline__ void ragged_pixel(uint32_t p, uint32_t w, uint32_t h, int& x, int& y) {
+    const uint32_t band = p / (4u * w), in_band = p - band * 4u * w;  // bands of four rows
+    const uint32_t th = min(4u, h - 4u * band);
+    const uint32_t col = in_band / (8u * th), in_tile = in_band - col * 8u * th;
+    const uint32_t tw = min(8u, w - 8u * col);
+    x = (int)(8u * col + in_tile % tw);
+    y = (int)(4u * band + in_tile / tw);
 }
 
 // tiled == 2: paths come in groups of g_s samples of every pixel; within a
@@ -57,6 +70,11 @@ __device__ __forceinline__ uint64_t tile2_index(const WaveDesc& W, uint32_t p, u
 __device__ __forceinline__ void wave_path(const WaveDesc& W, uint64_t g, int imgw, int& x, int& y, uint32_t& srel) {
     if (W.tiled == 2) {
         tile2_path(W, g, imgw, x, y, srel);
+        return;
+    }
+    if (W.tiled == 3) {
+        srel = (uint32_t)(g % (uint64_t)W.spp);
+        ragged_pixel((uint32_t)(g / (uint64_t)W.spp), (uint32_t)imgw, (uint32_t)(W.npix / imgw), x, y);
         return;
     }
     srel = (uint32_t)(g / (uint64_t)W.npix);

@@ -87,3 +87,29 @@ def test_query_spread_covers_every_ray(gpu_lib, port_lib, n):
     check(lib().nr_intersect_noalloc(S._h, m, *(x.ctypes.data for x in (oc, dc, tri, t, b1, b2))))
     for a, b in zip(got, (tri, t, b1, b2)):
         np.testing.assert_array_equal(a[:m], b)
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (1, 9, 3), (9, 1, 5), (7, 3, 3), (8, 4, 3), (9, 5, 1), (33, 18, 6), (64, 64, 12),
+                                     (101, 67, 7)])
+def test_pixel_order_gives_the_same_image(gpu_lib, w, h, spp):
+    """Frames or sample counts that tiles of a warp do not divide take all
+    samples of each pixel in turn, pixels in 8x4 tiles narrower and lower at
+    the edges: every pixel once, its samples added in sample order, also
+    where a wave ends between a pixel's samples."""
+    from nuray_gb300 import scenes
+    sc = scenes.small_scene(8)
+    S = Scene.from_arrays(sc["pos"], sc["mat"], sc["mats"], uv=sc["uv"], nrm=sc["nrm"], textures=sc["textures"],
+                          env_tex=sc["env_tex"], env_gain=sc["env_gain"])
+    p = (f"renderer=ptnee imgw={w} imgh={h} spp={spp} campos=0,14,34 cameuler=0,-20,0 camfov=50 camasp={w / h:.4f} "
+         "maxdepth=4")
+    ref = S.render(p + " tile=0")
+    for more in ("", " wave=1", " wave=50", " wave=777"):
+        if "wave=1" in more and w * h * spp > 3000:
+            continue
+        np.testing.assert_array_equal(S.render(p + more), ref, err_msg=more)
+    dl = np.random.default_rng(1).standard_normal((h, w, 3)).astype(np.float32)
+    a, ia = S.adjoint(p, dl, want_image=True)
+    b, ib = S.adjoint(p + " tile=0", dl, want_image=True)
+    np.testing.assert_array_equal(ia, ib)
+    # float atomics in any order: sums of up to 4 terms a path of either sign
+    np.testing.assert_allclose(a, b, rtol=1e-4, atol=1e-5 * max(1e-6, np.abs(a).max()))
