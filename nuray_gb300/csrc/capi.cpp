@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 #include <stdexcept>
@@ -222,6 +223,28 @@ bool reads_host(int device) {
         return false;
     }
     return a != 0 && b != 0;
+}
+
+struct HostSpan { const void* p; size_t bytes; };
+
+// Whether kernels may read `in` and write `out` where they lie. Staging copies
+// start at any byte, and a result that shares bytes with an input or with
+// another result is written after everything has been read, in the order of
+// the copies; a kernel wants whole floats and writes while it reads, so arrays
+// of either kind stay staged.
+bool in_place(std::initializer_list<HostSpan> in, std::initializer_list<HostSpan> out) {
+    auto at = [](const HostSpan& a) { return reinterpret_cast<uintptr_t>(a.p); };
+    auto apart = [&](const HostSpan& a, const HostSpan& b) { return at(a) + a.bytes <= at(b) || at(b) + b.bytes <= at(a); };
+    for (const HostSpan& a : in)
+        if (at(a) % 4) return false;
+    for (const HostSpan* a = out.begin(); a != out.end(); ++a) {
+        if (at(*a) % 4) return false;
+        for (const HostSpan& b : in)
+            if (!apart(*a, b)) return false;
+        for (const HostSpan* b = out.begin(); b != a; ++b)
+            if (!apart(*a, *b)) return false;
+    }
+    return true;
 }
 
 // Maps the pages of an output array that a kernel is going to write, its
@@ -1507,9 +1530,11 @@ int nr_intersect(nr_scene* s, int32_t n, const float* o, const float* d, int32_t
             // each of the six copies costs 7 us and more, and the kernel hides
             // the link behind the walks. us staged / in place: one ray 73 / 37,
             // 65,536 rays 189 / 112, 262,144 rays 337 / 155.
-            const bool host = !(flags & NR_PTR_DEVICE), staged = host && !s->host_access;
+            const size_t f3 = (size_t)n * 12, f1 = (size_t)n * 4;
+            const bool host = !(flags & NR_PTR_DEVICE);
+            const bool staged =
+                host && !(s->host_access && in_place({{o, f3}, {d, f3}}, {{tri, f1}, {t, f1}, {b1, f1}, {b2, f1}}));
             if (staged) {
-                size_t f3 = (size_t)n * 12, f1 = (size_t)n * 4;
                 s->scratch.ensure(2 * f3 + 4 * f1 + 6 * 256);  // six 256-byte aligned pieces
                 char* p = s->scratch.as<char>();
                 auto take = [&](size_t b) { char* r = p; p += (b + 255) & ~size_t(255); return r; };
@@ -1520,14 +1545,13 @@ int nr_intersect(nr_scene* s, int32_t n, const float* o, const float* d, int32_t
                 NR_CUDA(cudaMemcpyAsync(xd, d, f3, cudaMemcpyHostToDevice, st));
                 dO = xo; dD = xd;
             } else if (host) {
-                for (void* out : {(void*)tri, (void*)t, (void*)b1, (void*)b2}) touch_pages(out, (size_t)n * 4);
+                for (void* out : {(void*)tri, (void*)t, (void*)b1, (void*)b2}) touch_pages(out, f1);
             }
             NR_CUDA(cudaMemsetAsync(s->ps.counters + nr::CNT_ERR, 0, 4, st));
             nr::launch_intersect(scene_for(s, !(flags & NR_INTERSECT_EXHAUSTIVE)), n, dO, dD, dTri, dT, dB1, dB2,
                                  s->ps.counters + nr::CNT_ERR, st);
             NR_CUDA(cudaGetLastError());
             if (staged) {
-                size_t f1 = (size_t)n * 4;
                 NR_CUDA(cudaMemcpyAsync(tri, dTri, f1, cudaMemcpyDeviceToHost, st));
                 NR_CUDA(cudaMemcpyAsync(t, dT, f1, cudaMemcpyDeviceToHost, st));
                 NR_CUDA(cudaMemcpyAsync(b1, dB1, f1, cudaMemcpyDeviceToHost, st));
@@ -1860,8 +1884,9 @@ int nr_nrc_infer(nr_nrc* c, int32_t n, const float* x, float* out) {
         std::lock_guard<std::mutex> lk(c->mu);
         NR_CUDA(cudaSetDevice(c->device));
         const float* xf = nrc_rows_f32(c, n, x);
-        float* to = c->host_access ? out : c->out;
-        if (c->host_access) touch_pages(out, (size_t)n * 12);
+        const bool direct = c->host_access && in_place({{xf, (size_t)n * NRC_IN * 4}}, {{out, (size_t)n * 12}});
+        float* to = direct ? out : c->out;
+        if (direct) touch_pages(out, (size_t)n * 12);
         if (c->use_tc()) {
             nr::nrc_launch_forward_tc_f32(c->dev.wb, c->dev.params, xf, nullptr, nr::nrc_rows(n), to, c->num_sms,
                                           c->errbuf.as<uint32_t>(), c->stream, nullptr, c->tc_first_wait, nullptr);
@@ -1869,7 +1894,7 @@ int nr_nrc_infer(nr_nrc* c, int32_t n, const float* x, float* out) {
             nr::nrc_launch_to_bf16(xf, c->x, (size_t)n * NRC_IN, c->stream);
             nr::nrc_launch_forward(c->dev, c->x, nr::nrc_rows(n), to, nullptr, c->num_sms, c->stream);
         }
-        if (!c->host_access) NR_CUDA(cudaMemcpyAsync(out, c->out, (size_t)n * 12, cudaMemcpyDeviceToHost, c->stream));
+        if (!direct) NR_CUDA(cudaMemcpyAsync(out, c->out, (size_t)n * 12, cudaMemcpyDeviceToHost, c->stream));
         NR_CUDA(cudaMemcpyAsync(c->err_host, c->errbuf.p, 4, cudaMemcpyDeviceToHost, c->stream));
         NR_CUDA(cudaStreamSynchronize(c->stream));
         NR_CUDA(cudaGetLastError());
@@ -1884,7 +1909,7 @@ static int nrc_grad_impl(nr_nrc* c, int32_t n, const float* x, const float* y, f
         NR_CUDA(cudaSetDevice(c->device));
         const float* xf = nrc_rows_f32(c, n, x);
         const float* yd = y;
-        if (!c->host_access) {
+        if (!(c->host_access && in_place({{y, (size_t)n * 12}}, {}))) {
             NR_CUDA(cudaMemcpyAsync(c->y, y, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
             yd = c->y;
         }
