@@ -66,7 +66,10 @@ struct DevBuf;
 struct Budget {
     size_t cap = SIZE_MAX;
     size_t used = 0;
-    DevBuf* spare = nullptr;  // a buffer its user can do without: given up where another does not fit
+    // Buffers their users can do without, given up in this order where another
+    // does not fit: the ray sort's workspace, and the four-wide tree (*tree).
+    DevBuf* spare[2] = {};
+    const nr::WideNode** tree = nullptr;
 };
 
 struct DevBuf {
@@ -77,14 +80,16 @@ struct DevBuf {
     // touching the old buffer; if cudaMalloc fails the buffer is left empty,
     // so callers that cache sizes or pointers into it reset them first.
     void alloc(size_t n) {
-        if (budget && n > budget->cap - (budget->used - bytes) && !(drop_spare() && n <= budget->cap - (budget->used - bytes)))
+        auto over = [&]() { return budget && n > budget->cap - (budget->used - bytes); };
+        while (over() && drop_spare()) {}
+        if (over())
             throw NrError(NR_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes exceeds the scene's cap of " +
                                           std::to_string(budget->cap) + " bytes (" +
                                           std::to_string(budget->used - bytes) + " in use)");
         release();
         if (n == 0) return;
         cudaError_t e = cudaMalloc(&p, n);
-        if (e == cudaErrorMemoryAllocation && drop_spare()) {
+        while (e == cudaErrorMemoryAllocation && drop_spare()) {
             (void)cudaGetLastError();
             e = cudaMalloc(&p, n);
         }
@@ -94,9 +99,14 @@ struct DevBuf {
         if (budget) budget->used += n;
     }
     bool drop_spare() {
-        if (!budget || !budget->spare || budget->spare == this || !budget->spare->p) return false;
-        budget->spare->release();  // cudaFree waits for the device
-        return true;
+        if (!budget || this == budget->spare[0]) return false;  // the workspace makes do without before it takes the tree
+        for (DevBuf* b : budget->spare) {
+            if (!b || b == this || !b->p) continue;
+            if (b == budget->spare[1]) *budget->tree = nullptr;
+            b->release();  // cudaFree waits for the device
+            return true;
+        }
+        return false;
     }
     void release() {
         if (p) cudaFree(p);
@@ -190,7 +200,9 @@ struct nr_scene {
 
     nr_scene() {
         for (auto* b : all_bufs()) b->budget = &budget;
-        budget.spare = &sort_mem;
+        budget.spare[0] = &sort_mem;
+        budget.spare[1] = &wide;
+        budget.tree = &dev.wide;
     }
     std::vector<DevBuf*> all_bufs() {
         return {&nodes, &wide, &nodes_fast, &tri_geo, &tri_shade, &mats, &texels, &tex_info, &lights, &light_cdf, &light_guide,
@@ -449,7 +461,12 @@ void upload_scene(nr_scene* s) {
     upload(s->tri_shade, shade, st);
     upload(s->nodes, gn, st);
     upload(s->nodes_fast, gf, st);
-    upload(s->wide, wide, st);
+    try {
+        upload(s->wide, wide, st);
+    } catch (const NrError& e) {  // few rays then walk the other tree
+        if (e.code != NR_ERR_OOM) throw;
+        (void)cudaGetLastError();
+    }
     upload(s->mats, H.mats, st);
     upload(s->texels, texels, st);
     upload(s->tex_info, tinfo, st);
@@ -464,7 +481,7 @@ void upload_scene(nr_scene* s) {
 
     nr::DeviceScene& D = s->dev;
     D.nodes = s->nodes.as<nr::GpuNode>();
-    D.wide = s->wide.as<nr::WideNode>();  // null without nodes
+    D.wide = s->wide.as<nr::WideNode>();  // null without nodes or room
     D.nodes_fast = s->nodes_fast.as<nr::FastNode>();
     D.fast_origin_bound = 2.0f * A + 4.0f * E;
     D.tri_geo = s->tri_geo.as<float4>();
@@ -1430,7 +1447,6 @@ int nr_adjoint(nr_scene* s, const nr_camera* cam, const char* params, const floa
             NR_CUDA(cudaMemsetAsync(d_img, 0, b_img, st));
             NR_CUDA(cudaMemsetAsync(d_grad, 0, b_grad, st));
             nr::AdjArgs J;
-            J.S = scene_for(s, A.prune);
             J.pol = A.pol;
             J.cam = A.cam;
             J.film_h = nr::film_height(A.cam);
@@ -1452,6 +1468,7 @@ int nr_adjoint(nr_scene* s, const nr_camera* cam, const char* params, const floa
                 P1.tile = 0;
                 P1.tail = 0;  // the wavefront to the end, as the wavefront adjoint's first pass
                 run_waves(s, P1, npix, nullptr, A.sample0, nullptr, s->adj_L.as<float>(), nullptr, nullptr, nullptr);
+                J.S = scene_for(s, A.prune);
                 nr::launch_adjoint(J, d_dldi, d_grad, s->adj_L.as<float>(), s->num_sms, st);
                 launches = s->stats.kernel_launches + 1;
             } else {
