@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <initializer_list>
 #include <mutex>
 #include <new>
@@ -294,21 +295,6 @@ void upload_scene(nr_scene* s) {
     const int n = H.num_tris();
     cudaStream_t st = s->stream;
 
-    std::vector<float4> geo(3 * (size_t)n), shade(4 * (size_t)n);
-    for (int k = 0; k < n; ++k) {
-        int i = B.leaf_tris[k];
-        const float* p = &H.pos[9 * (size_t)i];
-        const float* t = &H.uv[6 * (size_t)i];
-        const float* nn = &H.nrm[9 * (size_t)i];
-        geo[3 * k] = make_float4(p[0], p[1], p[2], bits_f(i));
-        geo[3 * k + 1] = make_float4(p[3] - p[0], p[4] - p[1], p[5] - p[2], bits_f(H.mat[i]));
-        geo[3 * k + 2] = make_float4(p[6] - p[0], p[7] - p[1], p[8] - p[2], 0.0f);
-        shade[4 * k] = make_float4(nn[0], nn[1], nn[2], t[0]);
-        shade[4 * k + 1] = make_float4(nn[3], nn[4], nn[5], t[1]);
-        shade[4 * k + 2] = make_float4(nn[6], nn[7], nn[8], t[2]);
-        shade[4 * k + 3] = make_float4(t[3], t[4], t[5], bits_f(H.mat[i]));
-    }
-
     // internal nodes get consecutive GPU indices in depth-first order
     std::vector<int> gpu_index(B.nodes.size(), -1);
     int ng = 0;
@@ -336,24 +322,15 @@ void upload_scene(nr_scene* s) {
     // smaller index, and every leaf's triangles lie within the scene. A walk
     // then visits each node at most once and ends, and its stack holds at most
     // max_depth entries (checked against NR_STACK_LIMIT before the upload).
+    std::vector<int32_t> refs(2 * (size_t)ng);
+    for (int i = 0; i < ng; ++i) {
+        refs[2 * (size_t)i] = gn[i].d.x;
+        refs[2 * (size_t)i + 1] = gn[i].d.y;
+    }
     {
-        std::vector<int32_t> refs(2 * (size_t)ng);
-        for (int i = 0; i < ng; ++i) {
-            refs[2 * (size_t)i] = gn[i].d.x;
-            refs[2 * (size_t)i + 1] = gn[i].d.y;
-        }
         const std::string bad = nr::check_tree_refs(refs.data(), ng, n);
         if (!bad.empty()) throw NrError(NR_ERR_INVALID, bad);
     }
-
-    // each triangle's leaf, as the child it is
-    for (int k = 0; k < n; ++k) geo[3 * (size_t)k + 2].w = bits_f(-1);
-    for (int i = 0; i < ng; ++i)
-        for (int side = 0; side < 2; ++side) {
-            const int32_t r = side ? gn[i].d.y : gn[i].d.x;
-            if (r >= 0) continue;
-            for (int k = 0; k < nr::leaf_count(r); ++k) geo[3 * (size_t)(nr::leaf_first(r) + k) + 2].w = bits_f(2 * i + side);
-        }
 
     // The same nodes with every child box widened by delta for the one-FMA
     // box test without margin (fast_box). For a ray origin o with
@@ -372,6 +349,23 @@ void upload_scene(nr_scene* s) {
             E = std::max(E, 0.5f * (B.nodes[0].hi[k] - B.nodes[0].lo[k]));
         }
     const float delta = 4e-6f * (A + E) + 1e-30f;
+    // The four-wide tree, as long as the walk's stack holds it (a tree of chains
+    // may need more than its depth: then two children per node) and 32-bit
+    // byte offsets reach it. Built beside the rest (1M triangles: 12 ms).
+    auto build = [&]() {
+        std::vector<nr::WideNodeHost> w;
+        std::vector<float> box(12 * (size_t)ng);
+        for (int i = 0; i < ng; ++i) {
+            const nr::GpuNode& g = gn[i];
+            const float b[12] = {g.a.x, g.a.z, g.c.x, g.a.y, g.a.w, g.c.y, g.b.x, g.b.z, g.c.z, g.b.y, g.b.w, g.c.w};
+            std::copy(b, b + 12, &box[12 * (size_t)i]);
+        }
+        if (nr::build_wide(refs.data(), box.data(), ng, delta, 4, w) > NR_STACK_LIMIT)
+            nr::build_wide(refs.data(), box.data(), ng, delta, 2, w);
+        if (w.size() >= (size_t(1) << 25)) w.clear();
+        return w;
+    };
+    std::future<std::vector<nr::WideNodeHost>> wide = std::async(build);
     std::vector<nr::FastNode> gf(ng);
     for (int i = 0; i < ng; ++i) {
         const nr::GpuNode& g = gn[i];
@@ -381,24 +375,27 @@ void upload_scene(nr_scene* s) {
                              {0, 0}};
     }
 
-    // The four-wide tree, as long as the walk's stack holds it (a tree of chains
-    // may need more than its depth: then two children per node) and 32-bit
-    // byte offsets reach it.
-    std::vector<nr::WideNodeHost> wide;
-    {
-        std::vector<int32_t> refs(2 * (size_t)ng);
-        std::vector<float> box(12 * (size_t)ng);
-        for (int i = 0; i < ng; ++i) {
-            const nr::GpuNode& g = gn[i];
-            refs[2 * (size_t)i] = g.d.x;
-            refs[2 * (size_t)i + 1] = g.d.y;
-            const float b[12] = {g.a.x, g.a.z, g.c.x, g.a.y, g.a.w, g.c.y, g.b.x, g.b.z, g.c.z, g.b.y, g.b.w, g.c.w};
-            std::copy(b, b + 12, &box[12 * (size_t)i]);
+    std::vector<float4> geo(3 * (size_t)n), shade(4 * (size_t)n);
+    std::vector<int32_t> leaf(n, -1);  // each triangle's leaf, as the child it is
+    for (int i = 0; i < ng; ++i)
+        for (int side = 0; side < 2; ++side) {
+            const int32_t r = side ? gn[i].d.y : gn[i].d.x;
+            if (r < 0) std::fill_n(leaf.begin() + nr::leaf_first(r), nr::leaf_count(r), 2 * i + side);
         }
-        if (nr::build_wide(refs.data(), box.data(), ng, delta, 4, wide) > NR_STACK_LIMIT)
-            nr::build_wide(refs.data(), box.data(), ng, delta, 2, wide);
-        if (wide.size() >= (size_t(1) << 25)) wide.clear();
+    for (int k = 0; k < n; ++k) {
+        int i = B.leaf_tris[k];
+        const float* p = &H.pos[9 * (size_t)i];
+        const float* t = &H.uv[6 * (size_t)i];
+        const float* nn = &H.nrm[9 * (size_t)i];
+        geo[3 * k] = make_float4(p[0], p[1], p[2], bits_f(i));
+        geo[3 * k + 1] = make_float4(p[3] - p[0], p[4] - p[1], p[5] - p[2], bits_f(H.mat[i]));
+        geo[3 * k + 2] = make_float4(p[6] - p[0], p[7] - p[1], p[8] - p[2], bits_f(leaf[k]));
+        shade[4 * k] = make_float4(nn[0], nn[1], nn[2], t[0]);
+        shade[4 * k + 1] = make_float4(nn[3], nn[4], nn[5], t[1]);
+        shade[4 * k + 2] = make_float4(nn[6], nn[7], nn[8], t[2]);
+        shade[4 * k + 3] = make_float4(t[3], t[4], t[5], bits_f(H.mat[i]));
     }
+
     static_assert(sizeof(nr::WideNodeHost) == sizeof(nr::WideNode), "host and device node layouts");
 
     // emitters in loader order, weight = Triangle::area (twice the area)
@@ -461,12 +458,6 @@ void upload_scene(nr_scene* s) {
     upload(s->tri_shade, shade, st);
     upload(s->nodes, gn, st);
     upload(s->nodes_fast, gf, st);
-    try {
-        upload(s->wide, wide, st);
-    } catch (const NrError& e) {  // few rays then walk the other tree
-        if (e.code != NR_ERR_OOM) throw;
-        (void)cudaGetLastError();
-    }
     upload(s->mats, H.mats, st);
     upload(s->texels, texels, st);
     upload(s->tex_info, tinfo, st);
@@ -477,6 +468,13 @@ void upload_scene(nr_scene* s) {
     upload(s->env_weight, env_table.weight, st);
     upload(s->env_row_cdf, env_table.row_cdf, st);
     upload(s->env_col_cdf, env_table.col_cdf, st);
+    const std::vector<nr::WideNodeHost> wide_nodes = wide.get();
+    try {
+        upload(s->wide, wide_nodes, st);
+    } catch (const NrError& e) {  // few rays then walk the other tree
+        if (e.code != NR_ERR_OOM) throw;
+        (void)cudaGetLastError();
+    }
     NR_CUDA(cudaStreamSynchronize(st));
 
     nr::DeviceScene& D = s->dev;
