@@ -992,7 +992,7 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
             X.lo[k] = s->dev.root_lo[k];
             X.inv_ext[k] = ext > 0.f ? 1.0f / ext : 0.f;
         }
-        nrc_ensure_batch(s->nrc, std::max(s->nrc_tcap, cap));
+        nrc_ensure_batch(s->nrc, s->nrc_tcap);  // training rows; queries have their own table
     }
     // Where the order of a cache's training records decides what it learns from
     // them (several Adam steps on consecutive chunks; more records than the
