@@ -595,8 +595,8 @@ __global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_M
     warp_count(shadows, &P.counters[CNT_SHRAYS]);
 }
 
-// The two queues of a sorted bounce: blockIdx.y 0 writes the order of the
-// shadow queue, 1 the continuing paths into queue_out.
+// The queues of a sorted bounce: blockIdx.y 0 writes the order of the shadow
+// queue, 1 (where they are sorted too) the continuing paths into queue_out.
 __global__ void k_ray_order(PathState P) {
     const int which = blockIdx.y;
     const uint32_t n = which ? P.counters[CNT_OUT] : min(P.counters[CNT_SHADOW], (uint32_t)P.sh_cap);
@@ -844,16 +844,17 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
     const int most = g_num_sms * NR_SHADE_MINB * NR_SHADE_ROUNDS;
     if (shade_blocks > most) shade_blocks = most;
     PathState Q = P;
+    const int sorts = P.sort.place[1] ? 2 : (sorted ? 1 : 0);
     if (sorted) {  // shading appends the continuing paths beside, the sort moves them into queue_out
-        Q.queue_out = P.sort.queue;
-        for (int k = 0; k < 2; ++k) cudaMemsetAsync(P.sort.hist[k], 0, (size_t)P.sort.buckets() * 4, st);
+        if (sorts == 2) Q.queue_out = P.sort.queue;
+        for (int k = 0; k < sorts; ++k) cudaMemsetAsync(P.sort.hist[k], 0, (size_t)P.sort.buckets() * 4, st);
     }
     if (nrc) launch_shade<true>(Q, S, pol, capacity, capacity, shade_blocks, *nrc, st);
     else launch_shade<false>(Q, S, pol, capacity, max_count, shade_blocks, NrcCtx{}, st);
     if (sorted) {
-        k_ray_scan<<<dim3(P.sort.buckets() / 4096u, 2), 1024, 0, st>>>(P.sort);
-        k_ray_scan_parts<<<2, 1024, 0, st>>>(P.sort);
-        k_ray_order<<<dim3(g_num_sms * 4, 2), 256, 0, st>>>(P);
+        k_ray_scan<<<dim3(P.sort.buckets() / 4096u, sorts), 1024, 0, st>>>(P.sort);
+        k_ray_scan_parts<<<sorts, 1024, 0, st>>>(P.sort);
+        k_ray_order<<<dim3(g_num_sms * 4, sorts), 256, 0, st>>>(P);
     }
     if (ev) cudaEventRecord(ev[2], st);
     float4* tb = (nrc && nrc->direct) ? nrc->t_before : nullptr;

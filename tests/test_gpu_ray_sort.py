@@ -68,29 +68,29 @@ def test_without_room_for_the_sort_the_render_still_runs(gpu_lib):
         T.close()
 
 
-@pytest.mark.parametrize("more,sorts", [("", True), ("nrc=1", False), ("nrc=1 nrc_steps=1", True),
-                                        ("nrc=1 nrc_steps=1 nrc_train_depth=0", False), ("renderer=nrc", False)])
-def test_waves_whose_records_need_an_order_keep_it(gpu_lib, more, sorts):
+@pytest.mark.parametrize("more", ["", "nrc=1", "nrc=1 nrc_steps=1", "nrc=1 nrc_steps=1 nrc_train_depth=0", "renderer=nrc"])
+def test_waves_with_and_without_room_for_the_sort(gpu_lib, more):
     """Several Adam steps a wave take consecutive chunks of the training
-    records, and a full table keeps the first of them: such a wave is shaded
-    bounce by bounce in path order, without the sort's launches and without the
-    tail kernel in waves of this size."""
+    records, and a full table keeps the first of them: such a wave sorts its
+    shadow rays alone, and is shaded in path order without the tail kernel in
+    waves of this size. Every wave gives the unsorted one's first image, which
+    no training has touched."""
     from nuray_gb300.nrc import Cache
     S = _scene()
     c = Cache("seed=1")
     p = f"renderer=ptnee imgw=320 imgh=256 spp=52 {CAM} tail=0 "
     p = p.replace("renderer=ptnee", more) if "renderer" in more else p + more
     c.attach(S)
-    S.render(p)
+    a = S.render(p)
     with_order = S.stats()["kernel_launches"]
-    small = S.render(p.replace("spp=52", "spp=52 wave=4259840"))  # the same wave: all of it
-    assert np.all(np.isfinite(small))
     S.render(p + " profile=1")
     assert S.stats()["kernel_launches"] == with_order
-    # the same with room for the path state and the cache's records, but not for the sort (119 MB)
+    # the same with room for the path state and the cache's records, but not for the sort (67 MB and more)
     records = (4259840 * 64 + 16384 * 4 * 196) if "nrc" in more else 0
     T = _scene("max_device_bytes=%d" % _tight(320, 256, 4259840, 1, S, records + (16 << 20)))
     d = Cache("seed=1")
     d.attach(T)
-    T.render(p)
-    assert (with_order > T.stats()["kernel_launches"]) == sorts
+    b = T.render(p)
+    assert with_order > T.stats()["kernel_launches"]
+    if "renderer" not in more:  # whose first pass trains before the samples
+        np.testing.assert_array_equal(a, b)
