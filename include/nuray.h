@@ -125,7 +125,7 @@ typedef struct nr_stats {
     uint64_t rays;             /* extension rays (camera + continuation) */
     uint64_t shadow_rays;      /* NEE shadow rays */
     uint64_t waves;            /* wavefront batches */
-    uint64_t bounces;          /* trace/shade iterations over all waves */
+    uint64_t bounces;          /* trace/shade iterations over all waves (one launch of `tail` counts none) */
     uint64_t kernel_launches;  /* kernels launched by the call */
     uint64_t trace_launches;   /* of which closest-hit traversal */
     uint64_t nodes_visited;    /* BVH nodes visited by extension rays (count=1) */
@@ -293,9 +293,11 @@ int nr_intersect_noalloc(nr_scene* scene, int32_t n, const float* o, const float
  * in turn, pixels in 8x4 tiles. With tile_samples given, that tile or, where it
  * does not divide, as 1: 8x4 pixel tiles of one sample when imgw % 8 ==
  * 0 and imgh % 4 == 0; else or with 0: scanline order), live_sync (with
- * maxdepth: the bounce after which the live path count is read back each
- * bounce; -1, the default, 5 for waves of more than 2^22 paths and never
- * for smaller ones), tail (when
+ * maxdepth, in waves whose live path count is not read back anyway: the bounce
+ * after which it is, so that later bounces size their grids to the paths left;
+ * -1, the default, or 0: none. By default waves of more than 2^22 paths, waves
+ * without a depth limit and waves that tail=-1 may end early read it, one
+ * bounce behind), tail (when
  * one launch takes every live path to its end, tracing its light samples
  * inline: -1, the default, once a bounce starts with few paths; N > 0, in
  * waves of at most 2^22 paths after N wavefront bounces; 0 never; the image

@@ -735,12 +735,11 @@ struct RenderArgs {
     int tile;
     int tile_samples;     // 1, 2, 4, 8, 16 or 32
     bool tile_given;      // tile_samples came with the call
-    // With maxdepth: the bounces after which the live count is read back, so
-    // that later bounces size the shading grid to the paths left (0: never;
-    // -1, the default: 5 for waves of more than 2^22 paths, else never).
-    // 1M-triangle scene: 1080p x 64 spp 704.3 Mpaths/s with the readback
-    // against 699.0 without; 960x540 frames of 1 spp 2.789 ms with it,
-    // 2.735 without (the wait costs more than the grid saves).
+    // With maxdepth: the bounces after which the live count is read back where
+    // nothing else asks for it (waves of more than 2^22 paths and an automatic
+    // tail do), so that later bounces size the shading grid to the paths left;
+    // 0 or -1: none. The count is taken one bounce behind, so the device always
+    // has a bounce queued.
     int live_sync;
     // When k_tail takes every live path to its end in one launch: -1, the
     // default, by the live count (tail_limit); N > 0: in waves of at most 2^22
@@ -1032,7 +1031,7 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
     };
     NR_CUDA(cudaMemsetAsync(s->ps.counters, 0, nr::NUM_COUNTERS * 4, st));
     S.kernel_launches = 0;
-    const int live_sync = A.live_sync >= 0 ? A.live_sync : (cap > (1 << 22) ? 5 : 0);
+    const int live_sync = std::max(A.live_sync, 0);
     for (uint64_t base = 0; base < total; base += (uint64_t)cap) {
         if (cancel && *cancel == 0) throw NrError(NR_ERR_CANCELLED, "cancelled");
         nr::WaveDesc W;

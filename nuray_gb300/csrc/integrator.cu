@@ -522,10 +522,9 @@ static void launch_shade(const PathState& P, const DeviceScene& S, const Policy&
 #endif
 // Resident blocks per SM requested for the tail kernel. Its paths wait on
 // dependent traversal loads with few live lanes, so warps in flight pay more
-// than the registers' spills cost: 960x540 frames of 1 spp take 1.543 ms at 4
-// blocks (89 registers), 1.536 at 6, 1.463 at 8 (64 registers, 176 bytes
-// spilled), 1.459 at 10, 1.476 at 12 and 1.535 at 16 (40 and 32 registers,
-// kilobytes spilled).
+// than the registers' spills cost: 960x540 frames of 1 spp take 1.16 ms at 8
+// (64 registers) and 9 blocks; with a path per thread to its end 1.543 at 4 (89
+// registers), 1.536 at 6, 1.463 at 8, 1.459 at 10, 1.476 at 12 and 1.535 at 16.
 #ifndef NR_TAIL_MINB
 #define NR_TAIL_MINB 8
 #endif
