@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(1024) k_ray_scan_parts(RaySort s) {
         __syncthreads();
     }
 }
-__device__ __forceinline__ uint32_t ray_offset(const RaySort& s, int which, uint32_t q) {
-    const uint2 a = s.place[which][q];
+// Where the entry placed at (bucket, place) = a belongs.
+__device__ __forceinline__ uint32_t ray_offset(const RaySort& s, int which, uint2 a) {
     return s.hist[which][a.x] + s.part[which][a.x >> 12] + a.y;
 }
 
