@@ -642,12 +642,13 @@ void ensure_paths(nr_scene* s, int cap, int sh_mult = 1) {
 // samples, 8.3M 13.4 / 12.7; 1720 triangles, 8.4M 3.89 / 3.88; 36 triangles, 4.9M
 // 5.53 / 5.49. Bits an axis of the origin and of the direction: 132.7M paths
 // 4+3 130.0, 5+3 124.7, 6+2 124.5, 6+3 120.9; 8.3M 4+3 9.90, 5+3 9.67, 6+3 9.81.
-// Without room for the workspace the rays stay in queue order.
-// in_order (run_waves): the shadow rays alone, whose order nothing sees (1080p
-// x 64 spp with a cache of three steps: 117.3 ms without, 102.2 with).
+// Without room for the workspace the rays stay in queue order. in_order
+// (run_waves): sorted rays' paths are shaded in their own order all the same.
 void ensure_sort(nr_scene* s, int cap, int live, int sh_mult, bool in_order, nr::PathState& P) {
     nr::RaySort& R = P.sort;
-    R.input = R.place[1] ? 1 : 0;  // what the bounce before did
+    // what the bounce before did (the workspace has one size in a wave, so queue still holds its paths)
+    R.input = R.place[0] ? 1 : 0;
+    R.bucket_after = in_order ? R.input : 0;
     R.place[0] = R.place[1] = nullptr;
     if (live < 4000000 || s->dev.num_tris < 16384) return;
     R.origin_bits = cap >= (1 << 24) && s->dev.num_tris >= (1 << 19) ? 6 : 5;
@@ -658,8 +659,7 @@ void ensure_sort(nr_scene* s, int cap, int live, int sh_mult, bool in_order, nr:
     const size_t C = (size_t)cap, CS = C * (size_t)sh_mult, nb = R.buckets();
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     try {
-        s->sort_mem.ensure(2 * al(nb * 4) + 2 * al(nb / 4096 * 4) + al(CS * 8) + al(CS * 4) +
-                           (in_order ? 0 : al(C * 8) + al(C * 4)));
+        s->sort_mem.ensure(2 * al(nb * 4) + 2 * al(nb / 4096 * 4) + al(CS * 8) + al(CS * 4) + al(C * 8) + al(C * 4));
     } catch (const NrError& e) {
         if (e.code != NR_ERR_OOM) throw;
         (void)cudaGetLastError();
@@ -671,7 +671,6 @@ void ensure_sort(nr_scene* s, int cap, int live, int sh_mult, bool in_order, nr:
     for (auto& h : R.part) h = (uint32_t*)take(nb / 4096 * 4);
     R.place[0] = (uint2*)take(CS * 8);
     R.order = (int32_t*)take(CS * 4);
-    if (in_order) return;
     R.place[1] = (uint2*)take(C * 8);
     R.queue = (int32_t*)take(C * 4);
 }
@@ -1090,7 +1089,7 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
             S.bounces++;
             S.trace_launches++;
             S.kernel_launches += nr::bounce_launches(use_nrc ? cap : live, A.pol.envis != 0, s->dev.cat_mask) +
-                                 (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
+                                 (P.sort.place[0] ? nr::SORT_LAUNCHES : 0) + P.sort.bucket_after;
             // The count entering the next bounce, read back; the one asked for
             // a bounce earlier is taken now, while this bounce runs.
             const bool last = A.pol.maxdepth > 0 && bounce + 1 >= A.pol.maxdepth;
@@ -1255,7 +1254,7 @@ uint64_t adjoint_waves(nr_scene* s, const RenderArgs& A, int npix, const float* 
             ensure_sort(s, cap, live, s->sh_mult, false, P);
             nr::launch_bounce(P, D, pol1, cap, live, st, nullptr, false, nullptr);
             std::swap(P.queue_in, P.queue_out);
-            launches += nr::bounce_launches(live, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0);
+            launches += nr::bounce_launches(live, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0) + P.sort.bucket_after;
             if (!live_after(bounce, live)) break;
         }
         nr::launch_collect(s->ps, W, s->adj_L.as<float>(), A.spp, A.pol.imgw, st);

@@ -115,7 +115,8 @@ __device__ __forceinline__ void warp_count(uint32_t v, uint32_t* lohi) {
 #ifndef NR_SHADOW_MINB
 #define NR_SHADOW_MINB 10
 #endif
-// WALK: 0 exact; 1 fast, leaves postponed; 2 fast, for a sorted queue.
+// WALK: 0 exact; 1 fast, leaves postponed; 2 fast, for a sorted queue. Where the
+// order of the paths counts, a sorted queue's are bucketed by k_bucket.
 template <bool COUNT, int WALK>
 __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, DeviceScene S, int capacity) {
     const uint32_t n = P.counters[CNT_IN];
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, Devic
             const int tri = WALK ? closest_hit_fast<WALK == 1>(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr)
                                  : closest_hit_ww(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
+            if (P.sort.bucket_after) continue;
             int cat = CAT_MISS;
             if (tri >= 0) cat = S.mats[__float_as_int(__ldg(&S.tri_geo[3 * tri + 1]).w)].type;
             int pos = warp_append_keyed(cat, &P.counters[CNT_CAT]);
@@ -143,6 +145,44 @@ __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, Devic
     if (COUNT) {
         warp_count(nv, &P.counters[CNT_NODES]);
         warp_count(nt, &P.counters[CNT_TRIS]);
+    }
+}
+
+// The bucketing of k_trace in the order of the paths, for rays that were traced
+// in the order of the ray sort: a cache's training records keep the paths'
+// order. Bound by its gathers (the hit triangle's material); one counter update
+// per category and 1024 paths. PT+NRC of three steps, 1M triangles, 1080p x 64
+// spp: 99.9 ms, against 102.2 with only the shadow rays sorted and 117.3 with
+// neither. Waves without that need bucket in k_trace: shading reads slots next to each
+// other after k_bucket, but gains what k_bucket costs (122.4 against 123.6 ms).
+__global__ void __launch_bounds__(256) k_bucket(PathState P, DeviceScene S, int capacity) {
+    __shared__ uint32_t count[NUM_CAT], first[NUM_CAT];
+    const uint32_t n = P.counters[CNT_IN];
+    for (uint32_t b = blockIdx.x * 1024u; b < n; b += gridDim.x * 1024u) {
+        if (threadIdx.x < NUM_CAT) count[threadIdx.x] = 0u;
+        __syncthreads();
+        int slot[4], cat[4], pos[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t idx = b + 256u * k + threadIdx.x;
+            slot[k] = idx < n ? P.sort.queue[idx] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            cat[k] = CAT_MISS;
+            const int tri = slot[k] >= 0 ? __float_as_int(P.hit[slot[k]].w) : -1;
+            if (tri >= 0) cat[k] = S.mats[__float_as_int(__ldg(&S.tri_geo[3 * tri + 1]).w)].type;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (slot[k] >= 0) pos[k] = warp_append_keyed(cat[k], count);
+        __syncthreads();
+        if (threadIdx.x < NUM_CAT && count[threadIdx.x])
+            first[threadIdx.x] = atomicAdd(&P.counters[CNT_CAT + threadIdx.x], count[threadIdx.x]);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (slot[k] >= 0) P.sorted[(size_t)cat[k] * capacity + first[cat[k]] + pos[k]] = slot[k];
     }
 }
 
@@ -594,8 +634,8 @@ __global__ void __launch_bounds__(128, WALK == 3 ? NR_TAIL_MINB_WIDE : NR_TAIL_M
     warp_count(shadows, &P.counters[CNT_SHRAYS]);
 }
 
-// The queues of a sorted bounce: blockIdx.y 0 writes the order of the shadow
-// queue, 1 (where they are sorted too) the continuing paths into queue_out. Bound by its scattered
+// The two queues of a sorted bounce: blockIdx.y 0 writes the order of the
+// shadow queue, 1 the continuing paths into queue_out. Bound by its scattered
 // four-byte writes (132.7M paths' first bounce 3.6 ms); four entries a thread
 // and 32 blocks per SM in flight: 64 spp 123.7 ms, 124.0 with one entry and 4
 // blocks, 16 spp 32.67 / 32.76.
@@ -855,6 +895,7 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
         case 4: k_trace<true, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
         default: k_trace<true, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
     }
+    if (P.sort.bucket_after) k_bucket<<<std::max(1, std::min((max_count + 1023) / 1024, g_num_sms * 32)), 256, 0, st>>>(P, S, capacity);
     if (ev) cudaEventRecord(ev[1], st);
     // the shading kernels stride over their device counts; max_count (an
     // upper bound of their sum) and NR_SHADE_ROUNDS size the grids
@@ -863,17 +904,16 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
     const int most = g_num_sms * NR_SHADE_MINB * NR_SHADE_ROUNDS;
     if (shade_blocks > most) shade_blocks = most;
     PathState Q = P;
-    const int sorts = P.sort.place[1] ? 2 : (sorted ? 1 : 0);
     if (sorted) {  // shading appends the continuing paths beside, the sort moves them into queue_out
-        if (sorts == 2) Q.queue_out = P.sort.queue;
-        for (int k = 0; k < sorts; ++k) cudaMemsetAsync(P.sort.hist[k], 0, (size_t)P.sort.buckets() * 4, st);
+        Q.queue_out = P.sort.queue;
+        for (int k = 0; k < 2; ++k) cudaMemsetAsync(P.sort.hist[k], 0, (size_t)P.sort.buckets() * 4, st);
     }
     if (nrc) launch_shade<true>(Q, S, pol, capacity, capacity, shade_blocks, *nrc, st);
     else launch_shade<false>(Q, S, pol, capacity, max_count, shade_blocks, NrcCtx{}, st);
     if (sorted) {
-        k_ray_scan<<<dim3(P.sort.buckets() / 4096u, sorts), 1024, 0, st>>>(P.sort);
-        k_ray_scan_parts<<<sorts, 1024, 0, st>>>(P.sort);
-        k_ray_order<<<dim3(g_num_sms * ORDER_BLOCKS, sorts), 256, 0, st>>>(P);
+        k_ray_scan<<<dim3(P.sort.buckets() / 4096u, 2), 1024, 0, st>>>(P.sort);
+        k_ray_scan_parts<<<2, 1024, 0, st>>>(P.sort);
+        k_ray_order<<<dim3(g_num_sms * ORDER_BLOCKS, 2), 256, 0, st>>>(P);
     }
     if (ev) cudaEventRecord(ev[2], st);
     float4* tb = (nrc && nrc->direct) ? nrc->t_before : nullptr;

@@ -88,8 +88,8 @@ void launch_raygen(const PathState& P, const WaveDesc& W, const nr_camera& cam, 
 // trace + sort, shade (for bounces above 2^22 paths one kernel per shading
 // category the scene's materials can produce, else one for all; with a cache
 // by the wave's capacity), shadow, (envis: the environment samples' fold),
-// advance: bounce_launches(those paths, envis, scene category mask) kernels, and SORT_LAUNCHES more with P.sort (the
-// bounce's new rays sorted, ray_sort.cuh). ev (optional) receives 4 events.
+// advance: bounce_launches(those paths, envis, scene category mask) kernels, SORT_LAUNCHES more with P.sort (the
+// bounce's new rays sorted, ray_sort.cuh) and one more with P.sort.bucket_after (k_bucket). ev (optional) receives 4 events.
 constexpr int SORT_LAUNCHES = 3;
 constexpr int SHADE_SPLIT_MIN = 1 << 22;
 inline int bounce_launches(int paths, bool envis, uint32_t cat_mask) {
