@@ -68,26 +68,26 @@ def test_without_room_for_the_sort_the_render_still_runs(gpu_lib):
         T.close()
 
 
+@pytest.mark.parametrize("w,h,spp", [(320, 256, 52), (641, 399, 33)])
 @pytest.mark.parametrize("more", ["", "nrc=1", "nrc=1 nrc_steps=1", "nrc=1 nrc_steps=1 nrc_train_depth=0", "renderer=nrc"])
-def test_waves_with_and_without_room_for_the_sort(gpu_lib, more):
+def test_waves_with_and_without_room_for_the_sort(gpu_lib, more, w, h, spp):
     """Several Adam steps a wave take consecutive chunks of the training
-    records, and a full table keeps the first of them: such a wave sorts its
-    shadow rays alone, and is shaded in path order without the tail kernel in
-    waves of this size. Every wave gives the unsorted one's first image, which
-    no training has touched."""
+    records, and a full table keeps the first of them: such a wave is traced
+    sorted but bucketed and shaded in path order. Every wave gives the unsorted
+    one's first image, which no training has touched."""
     from nuray_gb300.nrc import Cache
     S = _scene()
     c = Cache("seed=1")
-    p = f"renderer=ptnee imgw=320 imgh=256 spp=52 {CAM} tail=0 "
+    p = f"renderer=ptnee imgw={w} imgh={h} spp={spp} {CAM} tail=0 "
     p = p.replace("renderer=ptnee", more) if "renderer" in more else p + more
     c.attach(S)
     a = S.render(p)
     with_order = S.stats()["kernel_launches"]
     S.render(p + " profile=1")
     assert S.stats()["kernel_launches"] == with_order
-    # the same with room for the path state and the cache's records, but not for the sort (67 MB and more)
-    records = (4259840 * 64 + 16384 * 4 * 196) if "nrc" in more else 0
-    T = _scene("max_device_bytes=%d" % _tight(320, 256, 4259840, 1, S, records + (16 << 20)))
+    # the same with room for the path state and the cache's records, but not for the sort (119 MB and more)
+    records = (w * h * spp * 64 + 16384 * 4 * 196) if "nrc" in more else 0
+    T = _scene("max_device_bytes=%d" % _tight(w, h, w * h * spp, 1, S, records + (16 << 20)))
     d = Cache("seed=1")
     d.attach(T)
     b = T.render(p)
