@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, Devic
 // in the order of the ray sort: a cache's training records keep the paths'
 // order. Bound by its gathers (the hit triangle's material); one counter update
 // per category and 1024 paths. PT+NRC of three steps, 1M triangles, 1080p x 64
-// spp: 99.9 ms, against 102.2 with only the shadow rays sorted and 117.3 with
+// spp: 98.4 ms, against 102.2 with only the shadow rays sorted and 116.5 with
 // neither. Waves without that need bucket in k_trace: shading reads slots next to each
 // other after k_bucket, but gains what k_bucket costs (122.4 against 123.6 ms).
 __global__ void __launch_bounds__(256) k_bucket(PathState P, DeviceScene S, int capacity) {
