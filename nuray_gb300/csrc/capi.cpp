@@ -1080,7 +1080,8 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
                 ev_kind.push_back(-1); ev_kind.push_back(0); ev_kind.push_back(1); ev_kind.push_back(2);
                 nev += 4;
             }
-            ensure_sort(s, cap, live, s->sh_mult, in_order, P);
+            // (the tail of a wave that keeps its order takes the paths as the queue has them)
+            ensure_sort(s, cap, in_order && cap <= nr::SHADE_SPLIT_MIN ? 0 : live, s->sh_mult, in_order, P);
             // large waves in pixel order: warps hold other rays than before, as in a sorted queue
             if (bounce == 0 && W.tiled == 3 && cap >= 4000000) P.sort.input = 1;
             nr::launch_bounce(P, D, A.pol, cap, live, st, A.profile ? evs : nullptr, A.count,

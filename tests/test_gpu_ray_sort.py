@@ -94,3 +94,17 @@ def test_waves_with_and_without_room_for_the_sort(gpu_lib, more, w, h, spp):
     assert with_order > T.stats()["kernel_launches"]
     if "renderer" not in more:  # whose first pass trains before the samples
         np.testing.assert_array_equal(a, b)
+
+
+def test_a_wave_whose_tail_keeps_its_order_is_not_sorted(gpu_lib):
+    """4.05M paths, several Adam steps: two bounces in path order, then the tail, which appends records as its queue stands."""
+    from nuray_gb300.nrc import Cache
+    launches = []
+    for more in ("nrc=1 nrc_steps=3", "nrc=1 nrc_steps=1"):
+        S = _scene()
+        c = Cache("seed=1")
+        c.attach(S)
+        S.render(f"renderer=ptnee imgw=320 imgh=256 spp=49 {CAM} {more} tail=2")
+        launches.append(S.stats()["kernel_launches"])
+    # 3 launches for each of two bounces' sorts; an Adam step is 4 launches
+    assert launches[0] == launches[1] - 2 * 3 + 2 * 4
