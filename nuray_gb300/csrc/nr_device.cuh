@@ -110,7 +110,7 @@ struct SlabRay {
     float ox, oy, oz;
     float dx, dy, dz;     // d + 1e-9f
     float rx, ry, rz;     // RN(1 / (d + 1e-9f))
-    float cx, cy, cz;     // RN(-o * r), for the one-FMA approximate quotient
+    float cx, cy, cz;     // RN(-o * r), for the one-FMA approximate quotient; NaN where r is infinite
     float abs_err;        // bound on |fma(b, r, c) - (b - o) r| from rounding c
 };
 __device__ __forceinline__ SlabRay make_slab_ray(f3 o, f3 d) {
@@ -118,7 +118,15 @@ __device__ __forceinline__ SlabRay make_slab_ray(f3 o, f3 d) {
     r.ox = o.x; r.oy = o.y; r.oz = o.z;
     r.dx = __fadd_rn(d.x, 1e-9f); r.dy = __fadd_rn(d.y, 1e-9f); r.dz = __fadd_rn(d.z, 1e-9f);
     r.rx = __frcp_rn(r.dx); r.ry = __frcp_rn(r.dy); r.rz = __frcp_rn(r.dz);
-    r.cx = -o.x * r.rx; r.cy = -o.y * r.ry; r.cz = -o.z * r.rz;
+    // A component of exactly -1e-9f leaves a denominator of 0 and an infinite
+    // r. qdiv's quotients are then NaN, which smax and smin pass over: the exact
+    // test leaves that axis out. With -o r one plane of a box that holds the
+    // origin would be infinite and the other NaN, and a minimum that drops the
+    // NaN puts both on one side; r - r is 0 for every finite r and NaN for this
+    // one, so the quotients below are NaN and their tests leave the axis out too.
+    r.cx = __fmaf_rn(-o.x, r.rx, __fsub_rn(r.rx, r.rx));
+    r.cy = __fmaf_rn(-o.y, r.ry, __fsub_rn(r.ry, r.ry));
+    r.cz = __fmaf_rn(-o.z, r.rz, __fsub_rn(r.rz, r.rz));
     // |c| * 2^-24 (rounding of c) with headroom: 2^-22
     r.abs_err = 2.4e-7f * fmaxf(fabsf(r.cx), fmaxf(fabsf(r.cy), fabsf(r.cz)));
     return r;
