@@ -349,21 +349,15 @@ void upload_scene(nr_scene* s) {
             E = std::max(E, 0.5f * (B.nodes[0].hi[k] - B.nodes[0].lo[k]));
         }
     const float delta = 4e-6f * (A + E) + 1e-30f;
-    // The four-wide tree, as long as the walk's stack holds it (a tree of chains
-    // may need more than its depth: then two children per node) and 32-bit
-    // byte offsets reach it. Built beside the rest (1M triangles: 12 ms).
+    // The four-wide tree (wide_tree), built beside the rest (1M triangles: 12 ms).
     auto build = [&]() {
-        std::vector<nr::WideNodeHost> w;
         std::vector<float> box(12 * (size_t)ng);
         for (int i = 0; i < ng; ++i) {
             const nr::GpuNode& g = gn[i];
             const float b[12] = {g.a.x, g.a.z, g.c.x, g.a.y, g.a.w, g.c.y, g.b.x, g.b.z, g.c.z, g.b.y, g.b.w, g.c.w};
             std::copy(b, b + 12, &box[12 * (size_t)i]);
         }
-        if (nr::build_wide(refs.data(), box.data(), ng, delta, 4, w) > NR_STACK_LIMIT)
-            nr::build_wide(refs.data(), box.data(), ng, delta, 2, w);
-        if (w.size() >= (size_t(1) << 25)) w.clear();
-        return w;
+        return nr::wide_tree(refs.data(), box.data(), ng, delta, NR_STACK_LIMIT);
     };
     std::future<std::vector<nr::WideNodeHost>> wide = std::async(build);
     std::vector<nr::FastNode> gf(ng);

@@ -841,4 +841,15 @@ int build_wide(const int32_t* refs, const float* box, int num_inner, float delta
     return need[0];
 }
 
+std::vector<WideNodeHost> wide_tree(const int32_t* refs, const float* box, int num_inner, float delta, int limit) {
+    std::vector<WideNodeHost> w;
+    // A ray whose direction is not a number passes every slot's test, unused
+    // ones too. At width 4 only nodes of leaves alone have any (a node opens
+    // inner children until it is full), two at most, and nothing lies below
+    // them: two entries more than build_wide counts. (At width 2 every node has
+    // two, three times its count: a tree of chains goes without.)
+    if (build_wide(refs, box, num_inner, delta, 4, w) + 2 > limit || w.size() >= (size_t(1) << 25)) w.clear();
+    return w;
+}
+
 }  // namespace nr

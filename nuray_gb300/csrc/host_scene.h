@@ -132,8 +132,11 @@ struct WideNodeHost {
 // its two children and opens the inner child of the largest surface until it
 // has `width`. Every box grows by delta on each side. Nodes come depth-first,
 // a parent before its children. Returns the deepest stack a depth-first walk
-// that pushes all hit children but one needs.
+// that pushes all hit children but one needs, unused slots never hit.
 int build_wide(const int32_t* refs, const float* box, int num_inner, float delta, int width,
                std::vector<WideNodeHost>& out);
+// The four-wide tree for walks without a stack test on `limit` entries, or
+// nothing where it does not fit them or 32-bit byte offsets do not reach it.
+std::vector<WideNodeHost> wide_tree(const int32_t* refs, const float* box, int num_inner, float delta, int limit);
 
 }  // namespace nr

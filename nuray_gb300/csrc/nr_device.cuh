@@ -842,7 +842,7 @@ __device__ __forceinline__ void wide_order(float& ta, int& ra, float& tb, int& r
 
 // Closest hit, nearest child first, a leaf at once. EXACT: leaves count by
 // their exact boxes (closest_hit_query's answer), else by the widened ones.
-// The host bounds the stack this needs (build_wide).
+// The host bounds the stack this needs, whatever the ray (wide_tree).
 template <bool EXACT>
 __device__ __forceinline__ int closest_hit_wide(const DeviceScene& S, f3 o, f3 d, float& best_t, float& best_b1,
                                                 float& best_b2) {
@@ -941,11 +941,14 @@ __device__ __forceinline__ bool any_hit_wide(const DeviceScene& S, f3 o, f3 d, f
 }
 
 // One ray of nr_intersect: closest_hit's answer by the faster walk where it
-// holds, the four-wide one if S has its nodes and the call asks for it.
+// holds, the four-wide one if S has its nodes and the call asks for it. Far
+// origins, and directions that are no numbers or beyond 1e30 (their
+// reciprocals near the denormals, where the widened boxes' margin is not shown
+// to cover the rounding), walk by closest_hit itself.
 template <bool WIDE>
 __device__ __forceinline__ int query_hit(const DeviceScene& S, f3 o, f3 d, float& t, float& b1, float& b2, uint32_t* err) {
     const float B = S.fast_origin_bound;
-    if (fabsf(o.x) <= B && fabsf(o.y) <= B && fabsf(o.z) <= B)
+    if (fabsf(o.x) <= B && fabsf(o.y) <= B && fabsf(o.z) <= B && fabsf(d.x) <= 1e30f && fabsf(d.y) <= 1e30f && fabsf(d.z) <= 1e30f)
         return WIDE ? closest_hit_wide<true>(S, o, d, t, b1, b2) : closest_hit_query(S, o, d, t, b1, b2);
     return closest_hit(S, o, d, t, b1, b2, err);
 }

@@ -91,7 +91,8 @@ struct DeviceScene {
     int32_t num_nodes;        // internal nodes
     float prune_k;            // subtrees entered beyond prune_k x the best hit are skipped (infinity: none)
     const FastNode* nodes_fast;  // the same nodes with every box widened, for the fast walk (trav=1)
-    const WideNode* wide;        // the four-wide tree, or null (a scene of one leaf, or more than 2^25 nodes)
+    const WideNode* wide;        // the four-wide tree, or null: a scene of one leaf, a tree that wide_tree leaves out,
+                                 // or no room on the device (at creation, or given up for a call's buffers)
     float fast_origin_bound;     // the fast walk is conservative for ray origins with every |coordinate| <= this
 };
 

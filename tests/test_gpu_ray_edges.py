@@ -1,6 +1,7 @@
 """Closest-hit queries with directions at the edge of the prepared ray's
 arithmetic: a component of exactly -1e-9f makes the box test's denominator
-d + 1e-9f zero."""
+d + 1e-9f zero; directions that are no numbers, or very long, walk by
+closest_hit."""
 import numpy as np
 import pytest
 
@@ -55,3 +56,93 @@ def test_denominator_of_zero(walks, axes):
     for got in _every_walk(walks, o, d):
         for a, b in zip(got, want):
             np.testing.assert_array_equal(a, b)
+
+
+def _rays(sc, n, seed):
+    r = np.random.default_rng(seed)
+    lo, hi = sc["pos"].reshape(-1, 3).min(0), sc["pos"].reshape(-1, 3).max(0)
+    return r.uniform(lo, hi, (n, 3)).astype(np.float32), r.standard_normal((n, 3)).astype(np.float32)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("axes", [(0,), (1,), (2,), (0, 1), (1, 2), (0, 1, 2)])
+def test_a_direction_that_is_no_number_hits_nothing(walks, axes, bad):
+    """Its determinant with any triangle is not finite. Rays beside it in the
+    same warp have their own answers."""
+    sc, S, _, _ = walks
+    o, d = _rays(sc, 3000, 7)
+    want = S.intersect(o, d)
+    d[::3, axes] = bad
+    for got in _every_walk(walks, o, d):
+        assert np.all(got[0][::3] == -1)
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a[1::3], b[1::3])
+            np.testing.assert_array_equal(a[2::3], b[2::3])
+
+
+def test_long_directions(walks):
+    sc, _, _, P = walks
+    o, d = _rays(sc, 3000, 8)
+    d *= (10.0 ** np.random.default_rng(9).uniform(28, 32, (3000, 1))).astype(np.float32)
+    want = P.intersect(o, d)
+    assert np.any(want[0] >= 0)
+    for got in _every_walk(walks, o, d):
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+
+
+def test_directions_of_zero(walks):
+    """The biased determinant is then 1e-6 for every triangle, and t says nothing
+    of where it lies: the exhaustive walk has the reference's answer, the
+    pruned ones end."""
+    sc, _, _, P = walks
+    o, d = _rays(sc, 3000, 10)
+    d[:] = 0
+    want = P.intersect(o, d)
+    got = _every_walk(walks, o, d)
+    for a, b, c in zip(got[-2], got[-1], want):
+        np.testing.assert_array_equal(a, c)
+        np.testing.assert_array_equal(b, c)
+
+
+@pytest.mark.parametrize("length", [31, 90])
+def test_tree_of_chains(gpu_lib, length):
+    """A tree (given to nr_scene_create_bvh) whose four-wide form fits the stack
+    at 31 levels and not at 90: the same answers, for a direction of NaN too."""
+    leaves = 4 * (length + 1)
+    r = np.random.default_rng(length)
+    x = np.arange(leaves)[:, None] * 0.5
+    c = np.concatenate([x, r.uniform(-1, 1, (leaves, 2))], 1)
+    pos = np.concatenate([c + [0, -0.5, -0.5], c + [0.1, 0.5, -0.5], c + [0.2, 0, 0.6]], 1).astype(np.float32)
+    lo, hi = pos.reshape(-1, 3, 3).min(1), pos.reshape(-1, 3, 3).max(1)
+    box, kids, first, count = [], [], [], []
+
+    def sub(a, b, chain):
+        me = len(box)
+        box.append(np.concatenate([lo[a:b].min(0), hi[a:b].max(0)]))
+        kids.append((-1, -1)), first.append(a), count.append(b - a)
+        if b - a > 1:
+            m = a + 4 if chain and b - a > 4 else (a + b) // 2
+            first[me] = count[me] = 0
+            kids[me] = (sub(a, m, False), sub(m, b, chain))
+        return me
+
+    sub(0, leaves, True)
+    tree = tuple(np.array(a, t) for a, t in zip((box, kids, first, count, np.arange(leaves)),
+                                                (np.float32, np.int32, np.int32, np.int32, np.int32)))
+    mats = [dict(type=0, c0=[0.5] * 3), dict(type=5, c0=[1.0] * 3)]
+    mat = np.zeros(leaves, np.int32)
+    mat[-1] = 1
+    S, T = Scene.from_arrays(pos, mat, mats, bvh=tree), Scene.from_arrays(pos, mat, mats)
+    o = r.uniform([-1, -1, -1], [leaves / 2, 1, 1], (2000, 3)).astype(np.float32)
+    d = r.standard_normal((2000, 3)).astype(np.float32)
+    d[::2, 1:] *= 0.05  # along the chain
+    d[::7] = np.nan
+    for a, b in zip(S.intersect(o, d), T.intersect(o, d)):
+        np.testing.assert_array_equal(a, b)
+    for a, b in zip(_noalloc(S, o, d), T.intersect(o, d)):
+        np.testing.assert_array_equal(a, b)
+    p = "renderer=ptnee imgw=16 imgh=8 spp=4 campos=" + f"{leaves / 2 - 1},0,4 " + "cameuler=0,0,0 camfov=60 camasp=2 maxdepth=4"
+    a, b = S.render(p), T.render(p)
+    assert np.all(np.isfinite(a))
+    np.testing.assert_allclose(a, b, rtol=1e-6, atol=1e-7)
