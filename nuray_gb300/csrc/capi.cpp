@@ -49,6 +49,7 @@ int guarded(F&& f) {
         f();
         return NR_OK;
     } catch (const NrError& e) {
+        (void)cudaGetLastError();  // reported now: not by the next call once more
         g_last_error = e.what();
         return e.code;
     } catch (const std::bad_alloc&) {
