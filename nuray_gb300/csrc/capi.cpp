@@ -677,6 +677,10 @@ void nrc_ensure_batch(nr_nrc* c, int m) {
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     size_t bytes = al(M * NRC_IN * 2) + al(M * 12) + al(M * 12) + al(4 * M * NRC_H * 2) + al(5 * M * NRC_H * 2) +
                    al(M * NRC_IN * 4);
+    // alloc frees the old scratch first: nothing may point into it if it then fails
+    c->batch_cap = 0;
+    c->x = c->acts = c->dz = nullptr;
+    c->y = c->out = c->xf = nullptr;
     c->batch.alloc(bytes);
     char* p = c->batch.as<char>();
     auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
