@@ -174,6 +174,7 @@ struct nr_scene {
     nr::HostScene host;
     nr::Bvh bvh;
     nr::DeviceScene dev{};
+    bool uploaded = false;  // dev's arrays are on the device
     DevBuf nodes, wide, nodes_fast, tri_geo, tri_shade, mats, texels, tex_info, lights, light_cdf, light_guide, light_mat;
     DevBuf adj_L;  // per-path radiance for the adjoint replay
     DevBuf adj_wave;  // per-slot state of the wavefront adjoint replay
@@ -449,6 +450,7 @@ void upload_scene(nr_scene* s) {
     }
     if (off > (size_t)INT32_MAX) throw NrError(NR_ERR_INVALID, "textures exceed 2^31 texels");
 
+    s->uploaded = false;  // dev points into arrays that are freed below
     upload(s->tri_geo, geo, st);
     upload(s->tri_shade, shade, st);
     upload(s->nodes, gn, st);
@@ -510,6 +512,7 @@ void upload_scene(nr_scene* s) {
         D.root_ref = R.left >= 0 ? 0 : nr::leaf_ref(R.first, R.count);
         for (int k = 0; k < 3; ++k) { D.root_lo[k] = R.lo[k]; D.root_hi[k] = R.hi[k]; }
     }
+    s->uploaded = true;
 }
 
 void finish_scene(nr_scene* s, const char* options, nr::Bvh* prebuilt = nullptr) {
@@ -772,6 +775,7 @@ void check_camera(const nr_scene* s, RenderArgs& A) {
 // The scene as the kernels of one call see it: the pruning factor of the
 // call's traversals.
 nr::DeviceScene scene_for(const nr_scene* s, bool prune) {
+    if (!s->uploaded) throw NrError(NR_ERR_OOM, "the scene's arrays did not fit the device when they were last replaced");
     nr::DeviceScene D = s->dev;
     D.prune_k = prune ? 1.0f + NR_PRUNE_MARGIN : INFINITY;
     return D;
@@ -1370,25 +1374,45 @@ int nr_scene_set_env(nr_scene* s, int32_t width, int32_t height, const float* rg
         std::lock_guard<std::mutex> lk(s->mu);
         NR_CUDA(cudaSetDevice(s->device));
         nr::HostScene& H = s->host;
-        // drop a previously attached environment that no material uses
+        const int32_t old_tex = H.env_tex;
+        const float old_gain = H.env_gain;
+        std::vector<float> old_data;  // of an environment that no material uses: dropped
+        std::vector<int32_t> old_wh;
         if (H.env_tex >= 0 && H.env_tex == (int)H.tex_wh.size() / 2 - 1) {
             bool used = false;
             for (const auto& m : H.mats) used = used || m.tex0 == H.env_tex || m.tex1 == H.env_tex;
             if (!used) {
                 size_t texels = (size_t)H.tex_wh[2 * H.env_tex] * H.tex_wh[2 * H.env_tex + 1];
+                old_data.assign(H.tex_data.end() - 3 * texels, H.tex_data.end());
+                old_wh.assign(H.tex_wh.end() - 2, H.tex_wh.end());
                 H.tex_data.resize(H.tex_data.size() - 3 * texels);
                 H.tex_wh.resize(H.tex_wh.size() - 2);
             }
         }
-        H.env_tex = -1;
-        if (width > 0) {
-            H.tex_wh.push_back(width);
-            H.tex_wh.push_back(height);
-            H.tex_data.insert(H.tex_data.end(), rgb, rgb + 3 * (size_t)width * height);
-            H.env_tex = (int)H.tex_wh.size() / 2 - 1;
+        const size_t kept_data = H.tex_data.size(), kept_wh = H.tex_wh.size();
+        try {
+            H.env_tex = -1;
+            if (width > 0) {
+                H.tex_wh.push_back(width);
+                H.tex_wh.push_back(height);
+                H.tex_data.insert(H.tex_data.end(), rgb, rgb + 3 * (size_t)width * height);
+                H.env_tex = (int)H.tex_wh.size() / 2 - 1;
+            }
+            H.env_gain = gain;
+            upload_scene(s);
+        } catch (...) {  // the scene as it was, on the device too: its arrays were being replaced
+            H.tex_data.resize(kept_data);
+            H.tex_wh.resize(kept_wh);
+            H.tex_data.insert(H.tex_data.end(), old_data.begin(), old_data.end());
+            H.tex_wh.insert(H.tex_wh.end(), old_wh.begin(), old_wh.end());
+            H.env_tex = old_tex;
+            H.env_gain = old_gain;
+            if (!s->uploaded) {
+                (void)cudaGetLastError();
+                try { upload_scene(s); } catch (const NrError&) {}  // scene_for reports it
+            }
+            throw;
         }
-        H.env_gain = gain;
-        upload_scene(s);
     });
 }
 
@@ -1408,6 +1432,7 @@ int nr_scene_set_materials(nr_scene* s, int32_t n, const nr_material* mats) {
         }
         std::lock_guard<std::mutex> lk(s->mu);
         NR_CUDA(cudaSetDevice(s->device));
+        const nr::DeviceScene D = scene_for(s, true);
         s->host.mats.assign(mats, mats + n);
         // On the device the materials stand in one table, and the emitters'
         // radiance in the light table as well; types, and with them everything
@@ -1415,7 +1440,7 @@ int nr_scene_set_materials(nr_scene* s, int32_t n, const nr_material* mats) {
         // scene instead: 6.7 ms for 200k triangles, against 0.03 ms.)
         NR_CUDA(cudaMemcpyAsync(s->mats.p, s->host.mats.data(), s->host.mats.size() * sizeof(nr_material), cudaMemcpyHostToDevice,
                                 s->stream));
-        nr::launch_set_emission(s->lights.as<float4>(), s->light_mat.as<int32_t>(), s->mats.as<nr_material>(), s->dev.num_lights,
+        nr::launch_set_emission(s->lights.as<float4>(), s->light_mat.as<int32_t>(), s->mats.as<nr_material>(), D.num_lights,
                                 s->stream);
         NR_CUDA(cudaGetLastError());
         NR_CUDA(cudaStreamSynchronize(s->stream));
@@ -1592,7 +1617,7 @@ int nr_intersect_noalloc(nr_scene* s, int32_t n, const float* o, const float* d,
                                               " rays per call (got " + std::to_string(n) + "); split the batch");
         std::lock_guard<std::mutex> lk(s->mu);
         NR_CUDA(cudaSetDevice(s->device));
-        std::string err = nr::noalloc_intersect(s->dev, s->device, s->stream, n, o, d, tri, t, b1, b2);
+        std::string err = nr::noalloc_intersect(scene_for(s, true), s->device, s->stream, n, o, d, tri, t, b1, b2);
         if (!err.empty()) throw NrError(err.rfind("traversal", 0) == 0 ? NR_ERR_DEVICE : NR_ERR_CUDA, err);
     });
 }
@@ -1999,7 +2024,7 @@ int nr_material_probe(nr_scene* s, int32_t mat, int32_t n, const float* wo, cons
         NR_CUDA(cudaMemcpyAsync(dwi, wi, f3, cudaMemcpyHostToDevice, st));
         NR_CUDA(cudaMemcpyAsync(duv, uv, f3, cudaMemcpyHostToDevice, st));
         NR_CUDA(cudaMemcpyAsync(du, u, f4, cudaMemcpyHostToDevice, st));
-        nr::launch_material_probe(s->dev, mat, n, dwo, dn, dwi, duv, du, df, dp, dws, st);
+        nr::launch_material_probe(scene_for(s, true), mat, n, dwo, dn, dwi, duv, du, df, dp, dws, st);
         NR_CUDA(cudaGetLastError());
         NR_CUDA(cudaMemcpyAsync(f, df, f3, cudaMemcpyDeviceToHost, st));
         NR_CUDA(cudaMemcpyAsync(pdf, dp, f1, cudaMemcpyDeviceToHost, st));
