@@ -906,9 +906,10 @@ RenderArgs parse_args(const nr_camera* cam, const char* params) {
 // pixel list is always in list order. Paths of one pixel start together and
 // their first bounces stay close: 1M triangles, 1080p, 9 samples 20.9 ms in
 // tiles of one sample, 19.7 in pixel order; 6 samples 14.4 (groups of two),
-// 13.7; 1919x1081 x 8 19.3 in scanlines, 17.7; 853x481 x 3 2.34, 2.25. in_order
-// (run_waves): never in pixel order.
-void wave_layout(const RenderArgs& A, bool has_pix_list, bool in_order, nr::WaveDesc& W) {
+// 13.7; 1919x1081 x 8 19.3 in scanlines, 17.7; 853x481 x 3 2.34, 2.25. by_samples:
+// never in pixel order, so that several waves are groups of samples of the whole
+// frame and not bands of it.
+void wave_layout(const RenderArgs& A, bool has_pix_list, bool by_samples, nr::WaveDesc& W) {
     W.tiled = 0;
     W.spp = A.spp;
     W.g_s = A.tile_samples;
@@ -916,7 +917,7 @@ void wave_layout(const RenderArgs& A, bool has_pix_list, bool in_order, nr::Wave
     W.g_h = 32 / (W.g_s * W.g_w);
     if (has_pix_list) return;
     const bool fits = A.pol.imgw % W.g_w == 0 && A.pol.imgh % W.g_h == 0 && A.spp % W.g_s == 0;
-    if (A.tile == 2 && !A.tile_given && !in_order && !(fits && (W.g_s >= 8 || W.g_s == A.spp))) W.tiled = 3;
+    if (A.tile == 2 && !A.tile_given && !by_samples && !(fits && (W.g_s >= 8 || W.g_s == A.spp))) W.tiled = 3;
     else if (A.tile == 2 && fits) W.tiled = 2;
     else if (A.tile >= 1 && A.pol.imgw % 8 == 0 && A.pol.imgh % 4 == 0) W.tiled = 1;
 }
@@ -1042,7 +1043,8 @@ void run_waves(nr_scene* s, const RenderArgs& A, int npix, const int32_t* dev_pi
         W.npix = npix;
         W.sample0 = (uint32_t)sample0;
         W.pix_xy = dev_pix;
-        wave_layout(A, dev_pix != nullptr, in_order, W);
+        // (what a cache learns from one wave shows in the next)
+        wave_layout(A, dev_pix != nullptr, in_order || (use_nrc && (uint64_t)cap < total), W);
         mark(-1);
         // queue_in / queue_out swap roles every bounce
         nr::PathState P = s->ps;
