@@ -431,6 +431,9 @@ __global__ void __launch_bounds__(128, NR_ADJ_SHADE_MINB) k_shade_adj(PathState 
         if (sg[i] != 0.f) atomicAdd(&grad[i], sg[i]);
 }
 
+// FAST: the walk of trav=1, whose answers the first pass's radiance holds (any
+// occluder decides, in whatever order); else the reference's boxes.
+template <bool FAST>
 __global__ void __launch_bounds__(128) k_shadow_adj(PathState P, DeviceScene S, AdjWave J, float* __restrict__ grad) {
     extern __shared__ float sg[];
     const int NG = S.num_mats * 7;
@@ -447,7 +450,7 @@ __global__ void __launch_bounds__(128) k_shadow_adj(PathState P, DeviceScene S, 
         const uint32_t idx = b + lane;
         if (idx < n) {
             const float4 o = P.sh_o[idx], d = P.sh_d[idx];
-            if (!any_hit_ww<true>(S, xyz(o), xyz(d), o.w, &P.counters[CNT_ERR])) {
+            if (!(FAST ? any_hit_fast(S, xyz(o), xyz(d), o.w) : any_hit_ww<true>(S, xyz(o), xyz(d), o.w, &P.counters[CNT_ERR]))) {
                 const int slot = __float_as_int(d.w);
                 const float4 c = P.sh_c[idx], r = P.rad[slot];
                 P.rad[slot] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.f);
@@ -474,7 +477,8 @@ int launch_adj_bounce_shading(const PathState& P, const DeviceScene& S, const Po
     const size_t smem = (size_t)S.num_mats * 7 * sizeof(float);
     k_shade_adj<<<num_sms * 8, 128, smem, st>>>(P, S, pol, capacity, J, vis, grad);
     if (vis) return 1;
-    k_shadow_adj<<<shadow_blocks, 128, smem, st>>>(P, S, J, grad);
+    if (pol.trav) k_shadow_adj<true><<<shadow_blocks, 128, smem, st>>>(P, S, J, grad);
+    else k_shadow_adj<false><<<shadow_blocks, 128, smem, st>>>(P, S, J, grad);
     return 2;
 }
 
@@ -531,7 +535,8 @@ __global__ void k_image_from_L(const float* __restrict__ Lbuf, int npix, int spp
 void adjoint_setup() {
     cudaFuncSetAttribute(k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_shade_adj, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_shadow_adj, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_shadow_adj<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_shadow_adj<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 void launch_image_from_L(const float* Lbuf, int npix, int spp, float* image_sum, cudaStream_t st) {

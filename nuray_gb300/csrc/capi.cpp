@@ -1258,6 +1258,8 @@ uint64_t adjoint_waves(nr_scene* s, const RenderArgs& A, int npix, const float* 
             P.hit = rec ? rec_hit + (size_t)bounce * C : s->ps.hit;
             P.vis = rec ? rec_vis + (size_t)bounce * C : nullptr;
             ensure_sort(s, cap, live, s->sh_mult, false, P);
+            // a bounce that pass 2 traces again, in an order of its own: by the walk whose hits the order leaves alone
+            if (!rec) P.sort.input = 1;
             nr::launch_bounce(P, D, pol1, cap, live, st, nullptr, false, nullptr);
             std::swap(P.queue_in, P.queue_out);
             launches += nr::bounce_launches(live, false, s->dev.cat_mask) + (P.sort.place[0] ? nr::SORT_LAUNCHES : 0) + P.sort.bucket_after;

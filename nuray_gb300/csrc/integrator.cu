@@ -115,8 +115,10 @@ __device__ __forceinline__ void warp_count(uint32_t v, uint32_t* lohi) {
 #ifndef NR_SHADOW_MINB
 #define NR_SHADOW_MINB 10
 #endif
-// WALK: 0 exact; 1 fast, leaves postponed; 2 fast, for a sorted queue. Where the
-// order of the paths counts, a sorted queue's are bucketed by k_bucket.
+// WALK: 0 exact, 1 fast, both with postponed leaves; 2 fast, 3 exact, whose hits
+// do not depend on the warp's other rays (a sorted queue; bounces that the
+// adjoint traces twice). Where the order of the paths counts, a sorted queue's
+// are bucketed by k_bucket.
 template <bool COUNT, int WALK>
 __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, DeviceScene S, int capacity) {
     const uint32_t n = P.counters[CNT_IN];
@@ -132,8 +134,10 @@ __global__ void __launch_bounds__(128, NR_TRACE_MINB) k_trace(PathState P, Devic
             int slot = P.queue_in[idx];
             f3 o = xyz(P.ray_o[slot]), d = xyz(P.ray_d[slot]);
             float t, b1, b2;
-            const int tri = WALK ? closest_hit_fast<WALK == 1>(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr)
-                                 : closest_hit_ww(S, o, d, t, b1, b2, COUNT ? &nv : nullptr, COUNT ? &nt : nullptr);
+            uint32_t *pv = COUNT ? &nv : nullptr, *pt = COUNT ? &nt : nullptr;
+            const int tri = WALK == 0   ? closest_hit_ww(S, o, d, t, b1, b2, pv, pt)
+                            : WALK == 3 ? closest_hit<false>(S, o, d, t, b1, b2, &P.counters[CNT_ERR], pv, pt)
+                                        : closest_hit_fast<WALK == 1>(S, o, d, t, b1, b2, pv, pt);
             P.hit[slot] = make_float4(t, b1, b2, __int_as_float(tri));
             if (P.sort.bucket_after) continue;
             int cat = CAT_MISS;
@@ -887,13 +891,15 @@ void launch_bounce(const PathState& P, const DeviceScene& S, const Policy& pol, 
                    cudaStream_t st, cudaEvent_t* ev, bool count, const NrcCtx* nrc) {
     const bool sorted = P.sort.place[0] != nullptr;
     if (ev) cudaEventRecord(ev[0], st);
-    switch ((count ? 3 : 0) + (pol.trav ? 1 + P.sort.input : 0)) {
+    switch ((count ? 4 : 0) + (pol.trav ? 1 + P.sort.input : 3 * P.sort.input)) {
         case 0: k_trace<false, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
         case 1: k_trace<false, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
         case 2: k_trace<false, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
-        case 3: k_trace<true, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
-        case 4: k_trace<true, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
-        default: k_trace<true, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 3: k_trace<false, 3><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 4: k_trace<true, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 5: k_trace<true, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        case 6: k_trace<true, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
+        default: k_trace<true, 3><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity); break;
     }
     if (P.sort.bucket_after) k_bucket<<<std::max(1, std::min((max_count + 1023) / 1024, g_num_sms * 32)), 256, 0, st>>>(P, S, capacity);
     if (ev) cudaEventRecord(ev[1], st);
@@ -947,8 +953,8 @@ void launch_tail(const PathState& P, const DeviceScene& S, const Policy& pol, in
 }
 
 void launch_trace(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, cudaStream_t st) {
-    if (pol.trav) k_trace<false, 1><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
-    else k_trace<false, 0><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
+    if (pol.trav) k_trace<false, 2><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
+    else k_trace<false, 3><<<g_trace_blocks, 128, 0, st>>>(P, S, capacity);
 }
 void launch_advance(uint32_t* counters, cudaStream_t st) { k_advance<<<1, 1, 0, st>>>(counters); }
 int shadow_grid() { return g_shadow_blocks; }

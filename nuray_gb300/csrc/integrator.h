@@ -102,7 +102,8 @@ void launch_nrc_apply(const PathState& P, const NrcCtx& C, const float* pred, in
 void launch_nrc_targets(const PathState& P, const NrcCtx& C, float* y, float clamp_max, cudaStream_t st);
 void launch_reset_counters(uint32_t* counters, cudaStream_t st);
 // The closest-hit + material-sort and advance steps alone, for wavefronts
-// that shade with kernels of their own (the adjoint replay).
+// that shade with kernels of their own (the adjoint replay): hits that do not
+// depend on the queue's order, as launch_bounce's with P.sort.input.
 void launch_trace(const PathState& P, const DeviceScene& S, const Policy& pol, int capacity, cudaStream_t st);
 void launch_advance(uint32_t* counters, cudaStream_t st);
 // Every live path of queue_in to its end in one launch; capacity (> 0) bounds

@@ -138,7 +138,8 @@ struct RaySort {
     int32_t origin_bits;  // per axis
     int32_t dir_bits;     // per axis of the octahedral map
     float cells_per_unit;
-    int32_t input;        // 1: queue_in is not in the order of the wave's warps (closest_hit_fast's POSTPONE)
+    int32_t input;        // 1: closest hits by a walk that does not look at the warp's other rays (queue_in is not in the
+                          // order of the wave's warps, or the bounce is traced twice)
     int32_t bucket_after; // 1: queue_in is sorted, queue holds its paths in their own order, and that order counts
     __host__ __device__ uint32_t buckets() const { return 1u << (3 * origin_bits + 2 * dir_bits); }
 };
