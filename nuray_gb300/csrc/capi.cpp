@@ -68,47 +68,61 @@ struct DevBuf;
 struct Budget {
     size_t cap = SIZE_MAX;
     size_t used = 0;
-    // Buffers their users can do without, given up in this order where another
-    // does not fit: the ray sort's workspace, and the four-wide tree (*tree).
-    DevBuf* spare[2] = {};
+    // Buffers their users can do without, given up where another does not fit:
+    // the ray sort's workspace, and the four-wide tree (*tree points to it), which
+    // stays away until the scene's arrays are next replaced.
+    DevBuf* sort = nullptr;
+    DevBuf* wide = nullptr;
     const nr::WideNode** tree = nullptr;
 };
+
+// Frees the ray sort's workspace of another scene on this device that no call
+// is using; false if there is none.
+bool free_idle_sort(const Budget* mine);
 
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     Budget* budget = nullptr;
-    // Replaces the buffer by one of n bytes. Over the cap it throws before
+    // Allocates n bytes. A request over the budget throws NR_ERR_OOM without
     // touching the old buffer; if cudaMalloc fails the buffer is left empty,
     // so callers that cache sizes or pointers into it reset them first.
     void alloc(size_t n) {
-        auto over = [&]() { return budget && n > budget->cap - (budget->used - bytes); };
-        while (over() && drop_spare()) {}
-        if (over())
+        auto over = [&](size_t freed) { return budget && n > budget->cap - (budget->used - bytes - freed); };
+        if (over(0)) drop(sort());
+        if (over(0) && wide() && !over(wide()->bytes)) drop(wide());
+        if (over(0))
             throw NrError(NR_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes exceeds the scene's cap of " +
                                           std::to_string(budget->cap) + " bytes (" +
                                           std::to_string(budget->used - bytes) + " in use)");
         release();
         if (n == 0) return;
         cudaError_t e = cudaMalloc(&p, n);
-        while (e == cudaErrorMemoryAllocation && drop_spare()) {
+        auto again = [&]() {
             (void)cudaGetLastError();
             e = cudaMalloc(&p, n);
-        }
+        };
+        if (e == cudaErrorMemoryAllocation && drop(sort())) again();
+        // (a workspace does without before it takes another's)
+        while (e == cudaErrorMemoryAllocation && !is_sort() && free_idle_sort(budget)) again();
+        size_t room = 0, all = 0;
+        if (e == cudaErrorMemoryAllocation && wide() && wide()->p && cudaMemGetInfo(&room, &all) == cudaSuccess &&
+            room + wide()->bytes >= n && drop(wide()))
+            again();
         if (e != cudaSuccess) p = nullptr;
         NR_CUDA(e);
         bytes = n;
         if (budget) budget->used += n;
     }
-    bool drop_spare() {
-        if (!budget || this == budget->spare[0]) return false;  // the workspace makes do without before it takes the tree
-        for (DevBuf* b : budget->spare) {
-            if (!b || b == this || !b->p) continue;
-            if (b == budget->spare[1]) *budget->tree = nullptr;
-            b->release();  // cudaFree waits for the device
-            return true;
-        }
-        return false;
+    bool is_sort() const { return budget && budget->sort == this; }
+    DevBuf* sort() const { return budget && !is_sort() ? budget->sort : nullptr; }
+    // what an allocation of this buffer may take the tree's room for
+    DevBuf* wide() const { return budget && !is_sort() && budget->wide != this ? budget->wide : nullptr; }
+    bool drop(DevBuf* b) {
+        if (!b || !b->p) return false;
+        if (b == budget->wide) *budget->tree = nullptr;
+        b->release();  // cudaFree waits for the device
+        return true;
     }
     void release() {
         if (p) cudaFree(p);
@@ -165,6 +179,19 @@ struct nr_nrc {
     }
 };
 
+namespace {
+// Every scene there is, for free_idle_sort. Never destroyed: scenes may outlive
+// the process's other statics.
+struct OpenScenes {
+    std::mutex mu;
+    std::vector<nr_scene*> list;
+};
+OpenScenes& open_scenes() {
+    static OpenScenes* all = new OpenScenes;
+    return *all;
+}
+}  // namespace
+
 struct nr_scene {
     std::mutex mu;
     int device = 0;
@@ -203,9 +230,11 @@ struct nr_scene {
 
     nr_scene() {
         for (auto* b : all_bufs()) b->budget = &budget;
-        budget.spare[0] = &sort_mem;
-        budget.spare[1] = &wide;
+        budget.sort = &sort_mem;
+        budget.wide = &wide;
         budget.tree = &dev.wide;
+        std::lock_guard<std::mutex> lk(open_scenes().mu);
+        open_scenes().list.push_back(this);
     }
     std::vector<DevBuf*> all_bufs() {
         return {&nodes, &wide, &nodes_fast, &tri_geo, &tri_shade, &mats, &texels, &tex_info, &lights, &light_cdf, &light_guide,
@@ -215,6 +244,11 @@ struct nr_scene {
     }
 
     ~nr_scene() {
+        {
+            std::lock_guard<std::mutex> lk(open_scenes().mu);
+            auto& l = open_scenes().list;
+            l.erase(std::find(l.begin(), l.end(), this));
+        }
         if (device >= 0) cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
         for (auto* b : all_bufs()) b->release();
@@ -227,6 +261,23 @@ struct nr_scene {
 };
 
 namespace {
+
+// A scene is in use while its lock is held; a call holds its own scene's lock
+// here (and may, from a progress callback, hold another's) and waits for no
+// other: no two calls can wait for each other.
+bool free_idle_sort(const Budget* mine) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lk(open_scenes().mu);
+    for (nr_scene* s : open_scenes().list) {
+        if (&s->budget == mine || s->device != device || !s->mu.try_lock()) continue;
+        std::lock_guard<std::mutex> theirs(s->mu, std::adopt_lock);
+        if (!s->sort_mem.p) continue;
+        s->sort_mem.release();
+        return true;
+    }
+    return false;
+}
 
 // Whether kernels on the device may use any host pointer (Grace and the GPU
 // share page tables over NVLink-C2C; elsewhere host arrays are staged).
