@@ -1677,7 +1677,7 @@ int nr_intersect_noalloc(nr_scene* s, int32_t n, const float* o, const float* d,
                                               " rays per call (got " + std::to_string(n) + "); split the batch");
         std::lock_guard<std::mutex> lk(s->mu);
         NR_CUDA(cudaSetDevice(s->device));
-        std::string err = nr::noalloc_intersect(scene_for(s, true), s->device, s->stream, n, o, d, tri, t, b1, b2);
+        std::string err = nr::noalloc_intersect(scene_for(s, true), s->device, s->num_sms, s->stream, n, o, d, tri, t, b1, b2);
         if (!err.empty()) throw NrError(err.rfind("traversal", 0) == 0 ? NR_ERR_DEVICE : NR_ERR_CUDA, err);
     });
 }

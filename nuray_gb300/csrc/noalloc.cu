@@ -82,7 +82,7 @@ std::string noalloc_prepare(int device) {
     return scratch_address(device, &base);
 }
 
-std::string noalloc_intersect(const DeviceScene& S, int device, cudaStream_t st, int n, const float* o, const float* d,
+std::string noalloc_intersect(const DeviceScene& S, int device, int num_sms, cudaStream_t st, int n, const float* o, const float* d,
                               int32_t* tri, float* t, float* b1, float* b2) {
     if (n < 0) return "n must be >= 0";
     if (n > NR_NOALLOC_MAX_RAYS)
@@ -110,8 +110,9 @@ std::string noalloc_intersect(const DeviceScene& S, int device, cudaStream_t st,
     if (e == cudaSuccess) e = cudaMemcpyAsync(so, o, f3, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(sd, d, f3, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return std::string("staging rays: ") + cudaGetErrorString(e);
-    // rays spread over 32 warps on each of 152 SMs, as launch_intersect spreads them
-    const int take = std::max(1, std::min(32, (n + 152 * 32 - 1) / (152 * 32))), blocks = (n + 4 * take - 1) / (4 * take);
+    // rays spread over 32 warps on each SM, as launch_intersect spreads them
+    const int warps = num_sms * 32, take = std::max(1, std::min(32, (n + warps - 1) / warps));
+    const int blocks = (n + 4 * take - 1) / (4 * take);
     if (S.wide) k_intersect_noalloc<true><<<blocks, 128, 0, st>>>(S, n, take, so, sd, stri, stt, sb1, sb2, serr);
     else k_intersect_noalloc<false><<<blocks, 128, 0, st>>>(S, n, take, so, sd, stri, stt, sb1, sb2, serr);
     e = cudaGetLastError();

@@ -19,7 +19,7 @@ namespace nr {
 // scene is created; returns "" or an error message.
 std::string noalloc_prepare(int device);
 
-std::string noalloc_intersect(const DeviceScene& S, int device, cudaStream_t st, int n, const float* o, const float* d,
-                              int32_t* tri, float* t, float* b1, float* b2);
+std::string noalloc_intersect(const DeviceScene& S, int device, int num_sms, cudaStream_t st, int n, const float* o,
+                              const float* d, int32_t* tri, float* t, float* b1, float* b2);
 
 }  // namespace nr
