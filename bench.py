@@ -15,9 +15,11 @@ value: paths / s with the scene resident and the image left on the device
 stream. e2e: the same render through nr_render with a pinned host output
 image, so the 24.9 MB device-to-host copy is inside the timed region.
 roofline: k_trace's algorithmic bytes (32 B per visited node, 36 B per
-tested triangle) per second against the measured copy bandwidth; beside it
-the issue roofline of k_trace and k_shadow (both issue-bound), and the whole
-path's bytes. c3 / c5_adjoint (after the timed steps, own clocks): frames of
+tested triangle) per second against the measured copy bandwidth. Most of them
+come from L1 and L2, so that fraction states a rate of work and not what
+bounds the kernel; beside it its DRAM bytes on the same scale, the issue
+roofline of k_trace and k_shadow (bound by the L1's data pipe and the issue
+slots), and the whole path's bytes. c3 / c5_adjoint (after the timed steps, own clocks): frames of
 the third workload (sky with importance sampling, textures, dielectrics, 256
 spp) and gradients of the inverse-rendering workload, timed the same way.
 time_to_relmse (not part of `value`): the metric's second half, plain PT
@@ -491,18 +493,21 @@ def main():
     trace_bytes = bytes_per_ray * rays
     achieved = trace_bytes / (trace_ms / 1e3) / 1e9 if trace_ms > 0 else None
     peak = pk.get("hbm_gbs", 6800.0)
-    roof = {"kernel": "k_trace (closest hit + material sort)", "bound": "hbm",
+    roof = {"kernel": "k_trace (closest hit + material sort)", "bound": "l1 data pipe / issue slots",
             "achieved": round(achieved, 1) if achieved else None, "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 3) if achieved else None, "peak_source": pk_kind,
             "traffic": None,
             "bytes_per_ray": round(bytes_per_ray, 1),
-            "bytes_formula": "32 B x nodes visited + 36 B x triangles tested per extension ray",
+            "bytes_formula": "32 B x nodes visited + 36 B x triangles tested per extension ray, "
+                             "most of them served by L1 and L2",
             "nodes_per_ray": round(cnt["nodes_visited"] / max(1, cnt["rays"]), 2),
             "tris_per_ray": round(cnt["tris_tested"] / max(1, cnt["rays"]), 2),
             "avg_launch_ms": round(trace_ms / max(1, trace_launches), 4),
             "share_of_step": round(trace_ms / ms, 3)}
     tr = NCU_CAPTURE["k_trace"]
     roof["traffic"] = round(tr["dram_bytes_per_ray"] * rays / max(1, trace_launches))
+    if trace_ms > 0:
+        roof["dram_frac"] = round(tr["dram_bytes_per_ray"] * rays / (trace_ms / 1e3) / 1e9 / peak, 3)
     roof["ncu_capture"] = {"source": NCU_CAPTURE["what"] + " (constants, not measured in this run)",
                            "dram_bytes_per_ray": tr["dram_bytes_per_ray"], "l2_hit_rate": tr["l2_hit_rate"],
                            "l1_hit_rate": tr["l1_hit_rate"],

@@ -286,7 +286,7 @@ int nr_intersect_noalloc(nr_scene* scene, int32_t n, const float* o, const float
  * the mean over all samples added so far), sample0 (index of the first
  * sample, default 0: renders of disjoint sample ranges are independent and
  * their films sum), tile (the order of a wave's paths; the image is the same
- * for every choice. 2, the default: each warp's 32 paths are tile_samples
+ * for every choice, with the exception under prune. 2, the default: each warp's 32 paths are tile_samples
  * consecutive samples of a tile of 32 / tile_samples pixels, tile_samples the
  * largest power of two up to 32 dividing spp, when the tile divides the image
  * and tile_samples is at least 8 or all of spp; else all samples of each pixel
@@ -301,11 +301,18 @@ int nr_intersect_noalloc(nr_scene* scene, int32_t n, const float* o, const float
  * one launch takes every live path to its end, tracing its light samples
  * inline: -1, the default, once a bounce starts with few paths; N > 0, in
  * waves of at most 2^22 paths after N wavefront bounces; 0 never; the image
- * is the same),
+ * is the same, with the exception under prune),
  * prune (1, the default: a traversal skips subtrees entered beyond 1.001 x
  * its best hit so far or its shadow ray's length; 0: every node whose box a
  * ray enters is visited, as the reference's exhaustive BVH::_traversal, for
- * the reference's hits on grazing rays as well; see nr_intersect),
+ * the reference's hits on grazing rays as well; see nr_intersect. With
+ * prune=1 a triangle that the reference reports nearer than its own box (its
+ * determinant is biased by 1e-6, which shows where twice a triangle's area
+ * seen along the ray is not far above that) wins or not by the order in which
+ * a walk meets it, and that order depends on tile, tail, the size of the wave
+ * and the room for the ray sort: about one path in 1e9 of a scene of 1M
+ * triangles 0.25 across ends elsewhere, many more of one a thousand times
+ * smaller. prune=0 has one image),
  * envis=1 (ptnee only, no reference counterpart: one environment light
  * sample per light-sampling vertex besides the area-light sample, weighted
  * against BSDF-sampled misses by the balance heuristic; the same expected
