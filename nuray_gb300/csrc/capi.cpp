@@ -1631,7 +1631,8 @@ int nr_intersect(nr_scene* s, int32_t n, const float* o, const float* d, int32_t
             // Host arrays are read and written in place where the device can:
             // each of the six copies costs 7 us and more, and the kernel hides
             // the link behind the walks. us staged / in place: one ray 73 / 37,
-            // 65,536 rays 189 / 112, 262,144 rays 337 / 155.
+            // 65,536 rays 189 / 112, 262,144 rays 337 / 155; in arrays of pages
+            // that the device has not met, 65,536 rays 302 / 145.
             const size_t f3 = (size_t)n * 12, f1 = (size_t)n * 4;
             const bool host = !(flags & NR_PTR_DEVICE);
             const bool staged =

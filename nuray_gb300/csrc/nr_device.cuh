@@ -529,7 +529,8 @@ __device__ __forceinline__ bool any_hit_ww(const DeviceScene& S, f3 o, f3 d, flo
 // Bound by the L1's data pipe and by issue slots at once (first-bounce shadow
 // rays: 84 % of the L1's wavefronts and 64 % of the issue slots), so a node
 // visit takes few, wide instructions: two 32-byte loads instead of four of
-// 16, six two-wide FMAs for the twelve quotients, three-operand min and max.
+// 16, six two-wide FMAs for the twelve quotients (three-operand min and max
+// the compiler forms by itself too).
 // 1M-triangle frame of 1080p x 64 spp against four 16-byte loads and scalar
 // FMAs: closest hit 78.2 -> 73.2 ms, shadow rays 46.3 -> 42.9, L1 wavefronts
 // of the first shadow bounce 333 M -> 284 M, warp instructions 982 M -> 835 M.
