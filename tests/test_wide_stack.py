@@ -9,6 +9,8 @@ import subprocess
 import numpy as np
 import pytest
 
+from nuray_gb300.build import _cuda_home
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "nuray_gb300", "csrc")
 OUT = os.path.join(ROOT, "tests", "_build")
@@ -38,7 +40,7 @@ def tree_lib():
     with open(src, "w") as f:
         f.write(SHIM)
     subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-shared", "-I", CSRC, "-I",
-                    os.path.join(ROOT, "include"), "-I", "/usr/local/cuda/include", src,
+                    os.path.join(ROOT, "include"), "-I", os.path.join(_cuda_home(), "include"), src,
                     os.path.join(CSRC, "host_scene.cpp"), os.path.join(CSRC, "image_io.cpp"),
                     os.path.join(CSRC, "jpeg.cpp"), "-o", lib, "-lpthread"], check=True)
     return ctypes.CDLL(lib)
